@@ -250,3 +250,89 @@ def tolerance(case):
     if case["kind"] in ("qk_hidden", "qk_heads"):
         return {"rel": 5e-3 if case["dtype"] == "bf16" else 1e-3}
     return {"rel": 1e-2 if case["dtype"] == "bf16" else 2e-3}
+
+
+# ---- the results in 64 bits -------------------------------------------------------------------------------------------------
+MOST_PAIRS = 6e10  # (query, key) pairs of all heads above which the 64-bit result takes too long
+
+
+def _selected(q, k, threshold, pq, bk, g, causal, chunk):
+    """Keep mask (query tiles, keys) of one head.  The pooled queries are 16-bit values by the operator's definition;
+    everything after them is 64-bit."""
+    s, n = k.shape[0], math.ceil(q.shape[0] / pq)
+    pad = n * pq - q.shape[0]
+    pooled = torch.nn.functional.pad(q.double(), (0, 0, 0, pad)).view(n, pq, D).sum(1)
+    rows = torch.full((n, 1), float(pq), dtype=torch.float64, device=q.device)
+    rows[-1] -= pad
+    pooled = ((pooled / rows).to(q.dtype).float() * (1.0 / math.sqrt(D))).to(q.dtype)
+    est = pooled.double() @ k.double().t()
+    blocks = math.ceil(s / bk)
+    groups = math.ceil(blocks / g)
+    tops = torch.full((n, groups * g * bk), -math.inf, dtype=torch.float64, device=q.device)
+    tops[:, :s] = est
+    if causal:
+        tops[:, :pq] = -math.inf
+    tops = tops.view(n, groups * g, bk).amax(-1).view(n, groups, g).cummax(-1).values.view(n, -1)
+    keep = est - math.log(threshold + 1e-9) >= tops.repeat_interleave(bk, dim=1)[:, :s]
+    if causal:  # the first tile and the diagonal one are dense; a chunk's every 64th tile loses most of the tile before its own
+        tile = torch.arange(n, device=q.device)
+        end = tile * pq
+        end = torch.where(tile % (chunk // pq) % 64 == 0, torch.minimum(end, (tile - 1) * pq + bk), end)[:, None]
+        key = torch.arange(s, device=q.device)[None]
+        tile = tile[:, None]
+        keep = (keep & (key >= pq) & (key < end)) | (key < pq) | ((key >= tile * pq) & (key < (tile + 1) * pq))
+    return keep
+
+
+def _attend(q, k, v, keep, pq, causal, row0=0):
+    """Softmax attention of one head's rows row0, row0 + 1, ...; keep: their tiles' keys, or None for all."""
+    out = torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    k, v = k.double(), v.double()
+    step = max(pq, int(1e8) // k.shape[0] // pq * pq)
+    for a in range(0, q.shape[0], step):
+        x = q[a:a + step].double() @ k.t() / math.sqrt(D)
+        n = x.shape[0]
+        if keep is not None:
+            x.masked_fill_(~keep[a // pq:(a + n + pq - 1) // pq].repeat_interleave(pq, dim=0)[:n], -math.inf)
+        if causal:
+            row = torch.arange(row0 + a, row0 + a + n, device=q.device)[:, None]
+            x.masked_fill_(torch.arange(k.shape[0], device=q.device)[None] > row, -math.inf)
+        out[a:a + n] = torch.softmax(x, dim=-1) @ v
+    return out
+
+
+def _normed_rotated(x, w, cos, sin, per_head, text):
+    """RMSNorm of the last dimension, then the rotation of (even, odd) pairs of every token that has angles."""
+    x = x.double()
+    x = x / torch.sqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    if per_head:
+        cos, sin = cos[:, ::2].double(), sin[:, ::2].double()
+        turned = x[:, :, :x.shape[2] - text]
+    else:
+        x = x.view(x.shape[0], x.shape[1], -1, D).transpose(1, 2)
+        cos, sin = cos.double(), sin.double()
+        turned = x[:, :, text:]
+    even, odd = turned[..., ::2], turned[..., 1::2]
+    turned[..., ::2], turned[..., 1::2] = even * cos - odd * sin, odd * cos + even * sin
+    return x
+
+
+def exact(case, seed):
+    kind, h, s = case["kind"], case["heads"], case["tokens"]
+    if kind not in ("qk_hidden", "qk_heads") and h * s * s > MOST_PAIRS:
+        return None
+    st = prepare(case, seed)
+    if kind in ("qk_hidden", "qk_heads"):
+        return tuple(_normed_rotated(x, w, st.cos, st.sin, kind == "qk_heads", case["text"]) for x, w in ((st.q, st.wq), (st.k, st.wk)))
+    out = torch.empty(st.q.shape, dtype=torch.float64, device="cuda")
+    begin, end = case.get("begin", 0), 0 if kind == "full" else case.get("end", s)
+    for i in range(h):
+        q, (k, v) = st.q[0, i].cuda(), (x[0, i // (h // case["kv_heads"])].cuda() for x in (st.k, st.v))
+        if end:
+            keep = _selected(q[:end], k[:end], case["threshold"], case["pq"], case["bk"], case["g"], case["causal"], case["chunk"])
+            out[0, i, :end] = _attend(q[:end], k[:end], v[:end], keep, case["pq"], case["causal"])
+        if begin:
+            out[0, i, :begin] = _attend(q[:begin], k, v, None, 64, True)
+        if end < s:
+            out[0, i, end:] = _attend(q[end:], k, v, None, 64, True, end)
+    return out
