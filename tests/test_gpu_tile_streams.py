@@ -1,0 +1,74 @@
+"""The attention kernels where tiles and chunks of very different lengths follow one another on one SM, against a plain
+fp32 softmax on the GPU.
+
+Tolerance: P and the result are rounded to 16 bits (relative 2^-9 in bf16), so an element is off by at most about
+2 * 2^-9 * max|v| plus its own rounding; max|v| of the normal draws below is under 5, hence 2e-2, and a tenth of it on average."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(autouse=True)
+def _needs_gpu(built_library):
+    if not torch.cuda.is_available():
+        pytest.fail("GPU tests need a CUDA device")
+
+
+def _close(got, ref):
+    err = (got.float() - ref).abs()
+    assert err.max().item() <= 2e-2 and err.mean().item() <= 2e-3, (err.max().item(), err.mean().item())
+
+
+@pytest.mark.parametrize("pq", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("longest,rise", [(2, 0.0), (300, 0.0), (300, 6.0)])
+def test_tiles_of_unequal_length(pq, dtype, longest, rise):
+    """More tiles than SMs several times over, with 0, 1, 2 ... chunks in no order.  ``rise``: scores that grow along the
+    list, so that the running maximum moves in every chunk and the partial results are rescaled."""
+    from vecattention_b200.api import _sparse_attn_bhsd
+    g = torch.Generator(device=DEV).manual_seed(5 + longest)
+    h, hkv, sk = 6, 2, 2000
+    nq = 900 // h
+    sq = nq * pq - 7
+    q = torch.randn(1, h, sq, 128, generator=g, device=DEV)
+    k = torch.randn(1, hkv, sk, 128, generator=g, device=DEV)
+    if rise:
+        q[..., 0] = 8.0
+        k[..., 0] = torch.linspace(0, rise * 11.3 / 8.0 * 4, sk, device=DEV)
+    q, k = q.to(dtype), k.to(dtype)
+    v = torch.randn(1, hkv, sk, 128, generator=g, device=DEV).to(dtype)
+    count = (torch.rand(1, h, nq, generator=g, device=DEV) ** 2 * (longest + 1)).int().clamp(max=longest)
+    cap = (longest + 3) // 4 * 4
+    order = torch.rand(h, nq, sk, generator=g, device=DEV).argsort(-1)[..., :cap].sort(-1).values
+    index = order.int()[None].contiguous()
+    out = _sparse_attn_bhsd(q, k, v, pq, None, None, count, index, False)
+    valid = torch.arange(cap, device=DEV) < count[0, :, :, None]
+    for i in range(h):
+        kk, vv = k[0, i // 3].float()[index[0, i].long()], v[0, i // 3].float()[index[0, i].long()]
+        qq = torch.nn.functional.pad(q[0, i].float(), (0, 0, 0, 7)).view(nq, pq, 128)
+        s = torch.bmm(qq, kk.transpose(1, 2)) / math.sqrt(128)
+        s.masked_fill_(~valid[i][:, None], -math.inf)
+        ref = torch.bmm(torch.softmax(s, -1).nan_to_num(0.0), vv).view(nq * pq, 128)[:sq]
+        _close(out[0, i], ref)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("s", [1, 127, 128, 129, 700, 2500])
+@pytest.mark.parametrize("bshd", [False, True])
+def test_dense_rows(dtype, s, bshd):
+    from vecattention_b200.dispatch import Full_prefill
+    g = torch.Generator(device=DEV).manual_seed(s)
+
+    def make(n):
+        x = torch.randn(2, s, n, 128, generator=g, device=DEV).to(dtype).transpose(1, 2)
+        return x if bshd else x.contiguous()
+
+    q, k, v = make(6), make(2), make(2)
+    out = Full_prefill(q, k, v)
+    ref = torch.nn.functional.scaled_dot_product_attention(q.float(), k.float().repeat_interleave(3, 1),
+                                                           v.float().repeat_interleave(3, 1), is_causal=True)
+    _close(out, ref)
