@@ -67,6 +67,29 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* tmap, int 
       : "memory");
 }
 
+// ---- cluster launch control: a running CTA takes over the work of a CTA of its grid that has not been launched yet ----
+// `res`: 16 bytes of shared memory (16-byte aligned) that receive the answer; 16 bytes complete on `bar`.  After an
+// answer that nothing was left the CTA must not ask again.
+__device__ __forceinline__ void clc_try_cancel(void* res, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_addr(res)),
+               "r"(smem_addr(bar))
+               : "memory");
+}
+// true: CTA `id` will not be launched, its work is the caller's
+__device__ __forceinline__ bool clc_answer(const void* res, uint3& id) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\tld.shared.b128 r, [%4];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\tselp.u32 %3, 1, 0, p;\n\t"
+      "mov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, %1, %2, _}, r;\n\t}"
+      : "=&r"(id.x), "=&r"(id.y), "=&r"(id.z), "=&r"(ok)
+      : "r"(smem_addr(res))
+      : "memory");
+  return ok != 0;
+}
+
 // generic-proxy writes to shared memory -> visible to the async proxy (UMMA operand reads)
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
