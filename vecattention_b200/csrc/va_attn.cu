@@ -27,7 +27,7 @@ int sparse_attn(const va_attn_args& a, cudaStream_t stream) {
   p.causal = a.causal; p.q_offset = a.q_offset;
   const float scale = a.softmax_scale > 0.f ? a.softmax_scale : 0.08838834764831845f;
   p.scale_log2 = scale * 1.4426950408889634f;
-  if (p.vis_on && p.vis_begin >= p.vis_end) {  // every row is dense: 128-row tiles on streamed K and V take 0.52 ms where
+  if (p.vis_on && p.vis_begin >= p.vis_end) {  // every row is dense: 128-row tiles on streamed K and V take 0.50 ms where
     // gathered 64-row tiles took 0.86 (28 query heads on 4 KV heads, 8192 tokens).  A composition with sparse rows keeps its
     // dense tiles in the 64-row launch: they are few, and a launch of their own would leave most SMs idle.
     AttnParams d = p;

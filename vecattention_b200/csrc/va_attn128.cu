@@ -25,8 +25,8 @@
 // and the tensor-memory latencies between them; both groups of a scheduler share its special-function unit), then, in the
 // sparse form, the gather beside them.  Measured on one B200 with the former kernel (P in shared memory, eight warps in
 // lockstep on one chunk, 64-row gathered tiles for dense rows): 32 heads x 32 K tokens causal at the reference's default
-// arguments 1.97 -> 1.73 ms for the whole operator; dense causal, 28 query heads on 4 KV heads, 8192 tokens, 0.855 -> 0.523 ms
-// (560 -> 920 TFLOP/s).
+// arguments 1.97 -> 1.73 ms for the whole operator; dense causal, 28 query heads on 4 KV heads, 8192 tokens, 0.855 -> 0.504 ms
+// (560 -> 950 TFLOP/s; 0.519 while the dense form too read a quarter of the scores twice for want of registers).
 #include "va_common.cuh"
 #include "va_sm100.cuh"
 #include "va_attn.cuh"
@@ -45,9 +45,12 @@ constexpr int kVStages = 2;
 constexpr int kThreads = 576;
 // Registers per thread: the kernel is launched with 96 (the most 18 warps can all have); the two producer warpgroups
 // hand 40 each back and the two softmax warpgroups take them: 256 * 56 + 256 * 136 + 64 * 96 = 576 * 96.
-constexpr int kProducerRegs = 56, kSoftmaxRegs = 136, kLaunchRegs = 96;
+// The dense kernel's producers only start TMA copies: they hand 72 each back, and a softmax thread can hold a whole row.
+constexpr int kLaunchRegs = 96;
+constexpr int kProducerRegs = 56, kSoftmaxRegs = 136, kDenseProducerRegs = 24, kDenseSoftmaxRegs = 168;
 // the softmax warps can only take what the producer warps hand back: the sum must fit the launch allocation
 static_assert(256 * kProducerRegs + 256 * kSoftmaxRegs + 64 * kLaunchRegs <= kThreads * kLaunchRegs, "setmaxnreg pool");
+static_assert(256 * kDenseProducerRegs + 256 * kDenseSoftmaxRegs + 64 * kLaunchRegs <= kThreads * kLaunchRegs, "setmaxnreg pool");
 constexpr size_t kSmem = 1024 + (size_t)kTileBytes * (1 + kKStages + kVStages);  // Q, K ring, V ring
 constexpr float kRescaleThreshold = 8.0f;                                        // log2 units
 
@@ -149,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
 
   if (warp >= 8 && warp < 16) {
     // ======================= gather producers (warps 8-11: K and the Q tile, warps 12-15: V) =======================
-    reg_dealloc<kProducerRegs>();
+    reg_dealloc<DENSE ? kDenseProducerRegs : kProducerRegs>();
     const bool is_v = warp >= 12;
     const int pt = is_v ? tid - 384 : tid - 256;
     const T* qb = static_cast<const T*>(p.q) + b * p.q_sb + h * p.q_sh;
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
     // a thread of either group owns a whole row.  The reference maximum of a row is one value shared by both groups
     // (m_row_s): the decision for chunk j starts from the value left by chunk j - 1, so all P tiles and O stay on one
     // scale.
-    reg_alloc<kSoftmaxRegs>();
+    reg_alloc<DENSE ? kDenseSoftmaxRegs : kSoftmaxRegs>();
     const int grp = warp >> 2, qtr = warp & 3;
     const uint32_t lane_base = (uint32_t)(qtr * 32) << 16;
     const int row = qtr * 32 + lane;
@@ -322,8 +325,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
         const int4 mk = *reinterpret_cast<const int4*>(mask_s[j & 7]);
         masked = (mk.x | mk.y | mk.z | mk.w) != 0;
       }
-      // ---- the row's maximum.  A whole row of 128 scores does not fit the registers: the first 32 are read again
-      // below, the other 96 stay (v[1..3]) ----
+      // ---- the row's maximum.  Beside the gather producers a whole row of 128 scores does not fit the registers: the
+      // first 32 are then read again below, the other 96 stay (v[1..3]) ----
       const uint32_t t_s = t_s0 + (uint32_t)(grp * 128) + lane_base;
       uint32_t v[4][32];
       float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -346,14 +349,26 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
       };
       tmem_ld32(t_s, v[0]);
       tmem_ld32(t_s + 32, v[1]);
-      tmem_wait_ld();
-      hide(0);
-      top(0);
-      tmem_ld32(t_s + 64, v[2]);
-      tmem_ld32(t_s + 96, v[3]);
-      hide(1);
-      top(1);
-      tmem_wait_ld();
+      if constexpr (DENSE) {
+        tmem_ld32(t_s + 64, v[2]);
+        tmem_ld32(t_s + 96, v[3]);
+        tmem_wait_ld();
+        tc_fence_before();
+        mbar_arrive(&bars.sempty[grp]);  // the S buffer has been read
+        hide(0);
+        top(0);
+        hide(1);
+        top(1);
+      } else {
+        tmem_wait_ld();
+        hide(0);
+        top(0);
+        tmem_ld32(t_s + 64, v[2]);
+        tmem_ld32(t_s + 96, v[3]);
+        hide(1);
+        top(1);
+        tmem_wait_ld();
+      }
       hide(2);
       hide(3);
       top(2);
@@ -410,12 +425,14 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
         }
       };
       expo(1);
-      tmem_ld32(t_s, v[0]);
-      tmem_wait_ld();
-      tc_fence_before();
-      mbar_arrive(&bars.sempty[grp]);  // the S buffer has been read
-      hide(0);
+      if constexpr (!DENSE) tmem_ld32(t_s, v[0]);
       expo(2);
+      if constexpr (!DENSE) {
+        tmem_wait_ld();
+        tc_fence_before();
+        mbar_arrive(&bars.sempty[grp]);  // the S buffer has been read
+        hide(0);
+      }
       expo(3);
       expo(0);
       const float2 la = halves(ls[0]), lb = halves(ls[1]);
