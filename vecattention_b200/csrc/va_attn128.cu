@@ -85,8 +85,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
   __shared__ float fin_s[256];                // [group * 128 + row]: row sums, added in the epilogue
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // causal tiles grow with their index: the longest are started first, so the grid's tail is made of short ones
-  const int tile = p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  int tile, h;
+  place(p, (int)gridDim.x, blockIdx.x, blockIdx.y, tile, h);
+  const int b = blockIdx.z;
   const int hkv = h / p.rep;
   int row0 = tile * PQ, row_end = p.sq;  // rows of the tile at or past row_end do not exist
   if constexpr (DENSE) {

@@ -13,7 +13,7 @@
 // its turn, its Q tile and first K and V rows are copied while the last chunks are worked on.  A CTA per tile spent 5-6 us a tile
 // on set-up, fill and drain, as much as six chunks of 128 keys.  Measured on one B200, whole operator, with the packed
 // arithmetic of the softmax: 28 query heads on 4 KV heads, 9001 tokens, causal 0.488 -> 0.403 ms; the same heads, 20011
-// tokens around a vision span, 1.23 -> 1.02 ms; 64 K tokens 6.61 -> 6.27 ms; 32 heads x 32 K tokens 3.54 -> 3.41 ms.
+// tokens around a vision span, 1.23 -> 1.02 ms (0.370 and 0.87 with their tiles listed by length); 64 K tokens 6.61 -> 6.27 ms; 32 heads x 32 K tokens 3.54 -> 3.41 ms.
 //
 // Warp roles (608 threads, one CTA per SM):
 //   warps 0-7  softmax: two groups of four warps (0-3, 4-7) take alternate chunks; inside a group
@@ -172,10 +172,9 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn64_kernel(const AttnPa
     bool more = true;
     for (int it = 0; !timed_out;) {
       bool have = more;
-      int row0 = 0, row_end = p.sq, tile = 0, dense = 0;
+      int row0 = 0, row_end = p.sq, tile = 0, head = 0, dense = 0;
       if (more) {
-        // causal tiles grow with their index: the longest are started first, so the grid's tail is made of short ones
-        tile = p.causal ? (int)(gridDim.x - 1 - id.x) : (int)id.x;
+        place(p, (int)gridDim.x, id.x, id.y, tile, head);
         // The tile's rows [row0, row_end).  Ordinarily tile t has rows 64 t ... ; in the vision-slice composition the
         // first p.nq tiles are the sparse tiles of rows [0, vis_end), cut to the rows from vis_begin on, and behind
         // them come dense tiles for rows [0, vis_begin) and for rows [vis_end, sq): all 64-key blocks up to the
@@ -204,7 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn64_kernel(const AttnPa
         Tile* t = &info_s[it % kInfo];
         if (!mbar_wait(&bars.iempty[it % kInfo], ((it / kInfo) & 1) ^ 1)) { timed_out = true; break; }
         if (more) {
-          const int64_t trow = dense ? 0 : ((int64_t)id.z * p.heads + id.y) * p.nq + tile;
+          const int64_t trow = dense ? 0 : ((int64_t)id.z * p.heads + head) * p.nq + tile;
           const int32_t* col = p.col_idx + trow * p.col_stride;
           int raw[8];
           // requested before the counts are known; a tile with dense blocks, which come first in slot order, fetches again
@@ -224,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn64_kernel(const AttnPa
 #pragma unroll
           for (int i = 0; i < 8; ++i) t->raw[i * 32 + lane] = raw[i];
           if (lane == 0) {
-            t->row0 = row0; t->row_end = row_end; t->h = (int)id.y; t->b = (int)id.z;
+            t->row0 = row0; t->row_end = row_end; t->h = head; t->b = (int)id.z;
             t->nblk = nblk; t->ncol = ncol; t->nchunks = (nblk * 64 + ncol + kChunk - 1) / kChunk; t->dense = dense;
             t->trow = trow;
           }
