@@ -1,0 +1,43 @@
+"""The rotation of qk_norm_rope rounds the double-precision result once, also where the fp32 arithmetic that serves nearly
+all pairs cannot decide: next to the middle between two 16-bit values, at magnitudes where products over- or underflow,
+at zeros and infinities.  Equality is exact; no tolerance."""
+import pytest
+import torch
+
+from oracle import vecattn_oracle as O
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("what", ["ordinary", "boundaries", "extremes"])
+def test_rotation_rounds_once(built_library, dtype, what):
+    if not torch.cuda.is_available():
+        pytest.fail("GPU tests need a CUDA device")
+    from vecattention_b200.preattn import qk_norm_rope
+    g = torch.Generator().manual_seed(11)
+    s, h = 700, 3
+    x = torch.randn(1, s, h * 128, generator=g)
+    cos, sin = torch.randn(s, 64, generator=g), torch.randn(s, 64, generator=g)
+    if what == "boundaries":
+        # results e + o * 2^-m exactly in the middle of two 16-bit values, or a last fp32 place beside it
+        bits = 8 if dtype == torch.bfloat16 else 11
+        x = 1 + torch.randint(0, 1 << (bits - 1), x.shape, generator=g) / float(1 << (bits - 1))
+        x[..., 1::2] = 1.0
+        cos[:] = 1.0
+        sin[:] = -(2.0 ** -bits) * (1 + torch.randint(-2, 3, sin.shape, generator=g) * 2.0 ** -23)
+    elif what == "extremes":
+        # every product is 0 or above 2^-149 (2^-50 of each factor, times normal draws, none under 2^-26 and 2^-18): the
+        # oracle's rounding goes through float32 and does not tell what underflows there to zero
+        low, high = (-50, 120) if dtype == torch.bfloat16 else (-14, 14)
+        x = x * 2.0 ** torch.randint(low, high + 1, x.shape, generator=g)
+        x[:, ::7, ::5] = 0.0
+        x[:, 3, 8:16] = float("inf")
+        cos = cos * 2.0 ** torch.randint(-50, 30, cos.shape, generator=g)
+        sin[::3] = 0.0
+        sin[1::5] *= 2.0 ** -50
+    x, cos, sin = x.to(dtype), cos.contiguous(), sin.contiguous()
+    q, k = qk_norm_rope(x.cuda(), x.cuda(), None, None, 1e-6, cos.cuda(), sin.cuda(), 0, heads=h)
+    ref = O.rope_interleaved(x.view(1, s, h, 128).transpose(1, 2), cos, sin)
+    for got in (q.cpu(), k.cpu()):
+        assert torch.equal(got.isnan(), ref.isnan())
+        assert torch.equal(got.nan_to_num(0.0), ref.nan_to_num(0.0))

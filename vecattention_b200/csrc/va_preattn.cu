@@ -26,6 +26,58 @@ __device__ __forceinline__ typename Elem<DT>::T from_double(double x) {
   else return __double2half(x);
 }
 
+// ---- the rotation of a pair, rounded once ----
+// x = a c - b s rounded once to the 16-bit type is what the double-precision expression gives.  Its conversions and the
+// rounding from double cost the kernel, which is bound by issue slots, more than the norm did, so nearly all pairs are
+// done in fp32 with the same result (40 heads, 75 600 tokens: 0.995 -> 0.827 ms, 3.15 -> 3.8 TB/s; a branch per pair instead of
+// one per piece of four: 0.886):
+//  * Kahan's product sum (w = b s; f = a c - w; t = f + (w - b s), both fma exact to their last rounding) is within
+//    1.5 units in the last place of x (Jeannerod, Louvet, Muller, "Further analysis of Kahan's algorithm for the accurate
+//    computation of 2 x 2 determinants", 2013) unless something over- or underflows: an overflow leaves an infinity or a
+//    NaN in t, and what an underflow can lose, 2^-149, is nothing beside an x of 2^-100 or more.
+//  * x then lies between t (1 - 2^-22) and t (1 + 2^-22) (2 to 4 units in the last place away, more where t is just
+//    below a power of two and x above it); if both round to the same 16-bit value, so does x.
+//  * Otherwise (a rounding boundary lies in between: one value in 10000 in bf16, in 1400 in fp16), or if some |t| is not between
+//    2^-100 and 2^100, the double-precision expression decides.
+constexpr float kTiny = 7.8886091e-31f, kHuge = 1.2676506e30f;  // 2^-100, 2^100
+template <int DT>
+__device__ __noinline__ uint32_t turn_exactly(float e, float o, float c, float s) {
+  using T = typename Elem<DT>::T;
+  const double ed = e, od = o, cd = c, sd = s;
+  const T r0 = from_double<DT>(ed * cd + (-od) * sd), r1 = from_double<DT>(od * cd + ed * sd);
+  return (uint32_t) * reinterpret_cast<const uint16_t*>(&r0) | ((uint32_t) * reinterpret_cast<const uint16_t*>(&r1) << 16);
+}
+// the four pairs (y[2 j], y[2 j + 1]) of a piece, turned by the angles with cosines c[j] and sines s[j], packed; one
+// branch for all of them
+template <int DT>
+__device__ __forceinline__ void turn(const float (&y)[8], const float (&c)[4], const float (&s)[4], uint32_t (&out)[4]) {
+  const uint64_t down = pair2(1.f - 2.38418579e-7f, 1.f - 2.38418579e-7f), up = pair2(1.f + 2.38418579e-7f, 1.f + 2.38418579e-7f);
+  uint32_t differ = 0, other[4];
+  float least = INFINITY, total = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float e = y[2 * j], o = y[2 * j + 1];
+    const uint64_t oe = pair2(o, e), ss = pair2(-s[j], s[j]), ns = pair2(s[j], -s[j]);
+    const uint64_t w = mul2(oe, ss), f = fma2(pair2(e, o), pair2(c[j], c[j]), w), over = fma2(oe, ns, w);  // over: w minus the exact product
+    const float2 fh = halves(f), oh = halves(over);
+    const float t0 = fh.x - oh.x, t1 = fh.y - oh.y;
+    least = fminf(fminf(least, fabsf(t0)), fabsf(t1));
+    total += fabsf(t0);
+    total += fabsf(t1);
+    const uint64_t t = pair2(t0, t1);
+    const float2 lo = halves(mul2(t, down)), hi = halves(mul2(t, up));
+    out[j] = Elem<DT>::pack(lo.x, lo.y);
+    other[j] = Elem<DT>::pack(hi.x, hi.y);
+    differ |= out[j] ^ other[j];
+  }
+  const bool plain = least >= kTiny && total <= kHuge;  // (false for a NaN)
+  if (differ != 0 || !plain) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (out[j] != other[j] || !plain) out[j] = turn_exactly<DT>(y[2 * j], y[2 * j + 1], c[j], s[j]);
+  }
+}
+
 // ---- the hidden-size form: W warps per token row ------------------------------------------------------------------
 // A row is taken by W = ceil(hidden / 1024) warps; a lane keeps its (up to) four 16-byte pieces packed in registers,
 // so every warp has its whole share of the row in flight at once, and the W warps add their partial sums through
@@ -34,7 +86,7 @@ __device__ __forceinline__ typename Elem<DT>::T from_double(double x) {
 // whole rows as fit eight warps.
 constexpr int NP = 4;  // pieces per lane
 template <int DT>
-__global__ void __launch_bounds__(256) qk_norm_rope_rows_kernel(const va_norm_rope_args a, int64_t rows, int W, int rows_per_cta) {
+__global__ void __launch_bounds__(256, 4) qk_norm_rope_rows_kernel(const va_norm_rope_args a, int64_t rows, int W, int rows_per_cta) {
   using T = typename Elem<DT>::T;
   __shared__ float part[8];  // [row of the CTA * W + warp of the row]
   const bool is_k = blockIdx.y == 1;
@@ -75,9 +127,17 @@ __global__ void __launch_bounds__(256) qk_norm_rope_rows_kernel(const va_norm_ro
     for (int i = 0; i < W; ++i) ss += part[rsub * W + i];  // the same order in every warp of the row
   }
   const float rstd = w ? 1.0f / sqrtf(ss / (float)hidden + a.eps) : 1.0f;  // no weight: no normalisation
+  const uint64_t rstd2 = pair2(rstd, rstd);
 
   const int rs = s - a.rope_skip;  // row of the cos / sin tables; the first rope_skip tokens are not rotated
-  const bool rotate = a.cos != nullptr && rs >= 0;
+  const bool rotate = live && a.cos != nullptr && rs >= 0;
+  float cc[4] = {}, sv[4] = {};
+  if (rotate) {  // a lane's pieces lie 32 W pieces apart, whole heads: all of them sit at the same place of their head
+    const int64_t at = (int64_t)rs * (kHeadDim / 2) + (lane & 15) * 4;
+    const float4 c = __ldg(reinterpret_cast<const float4*>(a.cos + at)), sn = __ldg(reinterpret_cast<const float4*>(a.sin + at));
+    cc[0] = c.x; cc[1] = c.y; cc[2] = c.z; cc[3] = c.w;
+    sv[0] = sn.x; sv[1] = sn.y; sv[2] = sn.z; sv[3] = sn.w;
+  }
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
     const int pc = wsub * 32 + lane + 32 * W * i;
@@ -91,8 +151,10 @@ __global__ void __launch_bounds__(256) qk_norm_rope_rows_kernel(const va_norm_ro
         for (int j = 0; j < 4; ++j) {
           const float2 f = Elem<DT>::unpack(ww[j]), v = Elem<DT>::unpack(xw[j]);
           // x_hat = x * rstd, y = x_hat * w, rounded to the 16-bit type as the norm kernel stores it
-          yv[2 * j] = Elem<DT>::to_float(Elem<DT>::from_float(__fmul_rn(__fmul_rn(v.x, rstd), f.x)));
-          yv[2 * j + 1] = Elem<DT>::to_float(Elem<DT>::from_float(__fmul_rn(__fmul_rn(v.y, rstd), f.y)));
+          const float2 n = halves(mul2(mul2(pair2(v.x, v.y), rstd2), pair2(f.x, f.y)));
+          const float2 y = Elem<DT>::unpack(Elem<DT>::pack(n.x, n.y));
+          yv[2 * j] = y.x;
+          yv[2 * j + 1] = y.y;
         }
       } else {
 #pragma unroll
@@ -104,17 +166,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope_rows_kernel(const va_norm_ro
       }
       uint32_t out[4];
       if (rotate) {
-        const int d0 = (pc * 8) % kHeadDim;  // position of the piece inside its head
-        const float4 c = __ldg(reinterpret_cast<const float4*>(a.cos + (int64_t)rs * (kHeadDim / 2) + d0 / 2));
-        const float4 sn = __ldg(reinterpret_cast<const float4*>(a.sin + (int64_t)rs * (kHeadDim / 2) + d0 / 2));
-        const float cc[4] = {c.x, c.y, c.z, c.w}, sv[4] = {sn.x, sn.y, sn.z, sn.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const double e = yv[2 * j], o = yv[2 * j + 1], cj = cc[j], sj = sv[j];
-          const T r0 = from_double<DT>(e * cj + (-o) * sj);
-          const T r1 = from_double<DT>(o * cj + e * sj);
-          out[j] = (uint32_t) * reinterpret_cast<const uint16_t*>(&r0) | ((uint32_t) * reinterpret_cast<const uint16_t*>(&r1) << 16);
-        }
+        turn<DT>(yv, cc, sv, out);
       } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j) out[j] = Elem<DT>::pack(yv[2 * j], yv[2 * j + 1]);
