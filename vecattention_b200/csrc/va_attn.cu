@@ -16,6 +16,9 @@ int sparse_attn(const va_attn_args& a, cudaStream_t stream) {
   p.k_sb = a.k.stride_b; p.k_sh = a.k.stride_h; p.k_ss = a.k.stride_s;
   p.v_sb = a.v.stride_b; p.v_sh = a.v.stride_h; p.v_ss = a.v.stride_s;
   p.o_sb = a.out.stride_b; p.o_sh = a.out.stride_h; p.o_ss = a.out.stride_s;
+  auto row_bytes = [](int64_t ss) { return ss >= -(1 << 30) && ss < (1 << 30) ? (int)(ss * 2) : 0; };
+  p.k_row_bytes = row_bytes(p.k_ss);
+  p.v_row_bytes = row_bytes(p.v_ss);
   p.blk_count = a.blk_idx ? a.blk_count : nullptr;
   p.blk_idx = a.blk_idx; p.blk_stride = a.blk_stride;
   p.col_count = a.col_count; p.col_idx = a.col_idx; p.col_stride = a.col_stride;

@@ -11,6 +11,7 @@ struct AttnParams {
   const void* v;
   void* out;
   int64_t q_sb, q_sh, q_ss, k_sb, k_sh, k_ss, v_sb, v_sh, v_ss, o_sb, o_sh, o_ss;
+  int k_row_bytes, v_row_bytes;  // k_ss, v_ss in bytes; 0: 32 bits do not hold them (or they are 0)
   const int32_t* blk_count;
   const int32_t* blk_idx;
   int64_t blk_stride;

@@ -12,8 +12,9 @@
 // score buffers and barriers run on over the tiles, the next tile's counts and first indices are in shared memory before
 // its turn, its Q tile and first K and V rows are copied while the last chunks are worked on.  A CTA per tile spent 5-6 us a tile
 // on set-up, fill and drain, as much as six chunks of 128 keys.  Measured on one B200, whole operator, with the packed
-// arithmetic of the softmax: 28 query heads on 4 KV heads, 9001 tokens, causal 0.488 -> 0.403 ms; the same heads, 20011
-// tokens around a vision span, 1.23 -> 1.02 ms (0.370 and 0.87 with their tiles listed by length); 64 K tokens 6.61 -> 6.27 ms; 32 heads x 32 K tokens 3.54 -> 3.41 ms.
+// arithmetic of the softmax: 28 query heads on 4 KV heads, 9001 tokens, causal 0.488 -> 0.368 ms; the same heads, 20011
+// tokens around a vision span, 1.23 -> 0.88 ms (both with their tiles listed by length); 64 K tokens 6.7 -> 6.2 ms; 32 heads x 32 K
+// tokens 3.6 -> 3.34 ms; 5 heads x 75 600 tokens 2.89 -> 2.72 ms.
 //
 // Warp roles (608 threads, one CTA per SM):
 //   warps 0-7  softmax: two groups of four warps (0-3, 4-7) take alternate chunks; inside a group
@@ -37,6 +38,8 @@
 #include "va_common.cuh"
 #include "va_sm100.cuh"
 #include "va_attn.cuh"
+
+#include <type_traits>
 
 namespace va {
 
@@ -250,115 +253,127 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn64_kernel(const AttnPa
   } else if (warp >= 8 && warp < 16) {
     // ======================= gather producers (warps 8-11: K and the Q tile, warps 12-15: V) =======================
     reg_dealloc<kProducerRegs>();
-    const bool is_v = warp >= 12;
-    const int pt = is_v ? tid - 384 : tid - 256;
-    // Copy geometry.  A warp covers two key rows per instruction: lanes 0-15 the sixteen 16-byte
-    // pieces of row rbase + 8 i, lanes 16-31 those of the next row.  Because the rows of one thread
-    // differ by multiples of 8, its swizzled piece position is the same in all of them and the
-    // shared-memory destinations are one base address plus i * 1024.
-    // Each lane fetches ONE key index per chunk (that of row rbase + 8 * (lane & 15)), two chunks
-    // ahead; the sixteen indices a thread needs are then exchanged through shared memory.
-    const int pw = (pt >> 5), hi = lane >> 4, c = lane & 15;
-    const int rbase = 2 * pw + hi;
-    const uint32_t dst_off = tile_off(128, rbase, c);
-    const int my_slot = rbase + 8 * c;
-    // All sixteen keys of this thread's rows, from the lanes that fetched them: through a small exchange array of
-    // the warp (one store and four 16-byte loads per thread instead of sixteen shuffles; two buffers, so the
-    // next chunk's stores cannot overtake this chunk's loads).
-    int* xk = xk_s[warp - 8][0];
-    uint32_t g = 0, n = 0;
-    int stage = 0;           // ring position of the chunk, and how often the ring has gone round (mod 2)
-    uint32_t round = 0;
-    for (int it = 0; !timed_out; ++it) {
-      const Tile* t = tile_info(it);
-      if (t == nullptr) break;
-      const int nchunks = t->nchunks, nblk = t->nblk, ncol = t->ncol, row0 = t->row0, row_end = t->row_end, h = t->h, b = t->b;
-      const bool dense = VIS && t->dense;
-      const int64_t trow = t->trow;
-      int raw0 = t->raw[my_slot], raw1 = t->raw[kChunk + my_slot];
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&bars.iempty[it % kInfo]);
-        if (warp == 8) mbar_arrive(&bars.begun);
-      }
-      if (nchunks < 0) break;
-      if (nchunks == 0) continue;
-      const int hkv = h / p.rep;
-      const T* src = (is_v ? static_cast<const T*>(p.v) + b * p.v_sb + hkv * p.v_sh
-                           : static_cast<const T*>(p.k) + b * p.k_sb + hkv * p.k_sh) + c * 8;
-      const int64_t stride = is_v ? p.v_ss : p.k_ss;
-      const int32_t* blk = dense ? nullptr : p.blk_idx + trow * p.blk_stride;  // no table: blocks 0, 64, 128, ...
-      const int32_t* col = p.col_idx + trow * p.col_stride;
-      if (!is_v) {
-        // the Q buffer is free once the last S product of the tile before the previous one has been computed
-        if (!mbar_wait(&bars.qempty[n & 1], ((n >> 1) & 1) ^ 1)) { timed_out = true; break; }
-        const T* qb = static_cast<const T*>(p.q) + b * p.q_sb + h * p.q_sh;
-        unsigned char* qt = q_s + (n & 1) * kQTile;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {  // Q tile: rows beyond the sequence are zero
-          const int pce = pt + i * 128, r = pce >> 4, cq = pce & 15;
-          const bool ok = row0 + r < row_end;
-          cp_async16(smem_addr(qt + tile_off(64, r, cq)), qb + (int64_t)(ok ? row0 + r : 0) * p.q_ss + cq * 8, ok);
+    // One body, compiled for K and for V: the loop has few registers and sets the pace of the kernel.  With the choice made
+    // at run time and 64-bit row offsets it spilled: 5 heads x 75 600 tokens 2.92 ms instead of 2.72, 32 heads x 32 K tokens
+    // 3.46 instead of 3.34.
+    auto produce = [&](auto is_v_c) {
+      constexpr bool is_v = decltype(is_v_c)::value;
+      const int pt = is_v ? tid - 384 : tid - 256;
+      // Copy geometry.  A warp covers two key rows per instruction: lanes 0-15 the sixteen 16-byte
+      // pieces of row rbase + 8 i, lanes 16-31 those of the next row.  Because the rows of one thread
+      // differ by multiples of 8, its swizzled piece position is the same in all of them and the
+      // shared-memory destinations are one base address plus i * 1024.
+      // Each lane fetches ONE key index per chunk (that of row rbase + 8 * (lane & 15)), two chunks
+      // ahead; the sixteen indices a thread needs are then exchanged through shared memory.
+      const int pw = (pt >> 5), hi = lane >> 4, c = lane & 15;
+      const int rbase = 2 * pw + hi;
+      const uint32_t dst_off = tile_off(128, rbase, c);
+      const int my_slot = rbase + 8 * c;
+      // All sixteen keys of this thread's rows, from the lanes that fetched them: through a small exchange array of
+      // the warp (one store and four 16-byte loads per thread instead of sixteen shuffles; two buffers, so the
+      // next chunk's stores cannot overtake this chunk's loads).
+      int* xk = xk_s[warp - 8][0];
+      uint32_t g = 0, n = 0;
+      int stage = 0;           // ring position of the chunk, and how often the ring has gone round (mod 2)
+      uint32_t round = 0;
+      for (int it = 0; !timed_out; ++it) {
+        const Tile* t = tile_info(it);
+        if (t == nullptr) break;
+        const int nchunks = t->nchunks, nblk = t->nblk, ncol = t->ncol, row0 = t->row0, row_end = t->row_end, h = t->h, b = t->b;
+        const bool dense = VIS && t->dense;
+        const int64_t trow = t->trow;
+        int raw0 = t->raw[my_slot], raw1 = t->raw[kChunk + my_slot];
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&bars.iempty[it % kInfo]);
+          if (warp == 8) mbar_arrive(&bars.begun);
         }
-        cp_async_arrive_noinc(&bars.qfull[n & 1]);
-      }
-      // K and V have producer warps of their own, so neither copy waits behind the other's stage:
-      // a K stage is free as soon as S has been computed from it, a V stage only after the PV
-      // product.  Raw index loads run two chunks ahead and are only interpreted at the top of a
-      // later iteration, so the in-order warp never stalls on them.
-      // a tile without dense blocks (every non-causal tile): slot s is entry s of the column list
-      const bool plain = nblk == 0;
-      for (int j = 0; j < nchunks; ++j, ++g) {
-        const int slot = j * kChunk + my_slot;
-        int key;
-        if (plain) {
-          key = (slot < ncol && (unsigned)raw0 < (unsigned)p.sk) ? raw0 : -1;
-          raw0 = raw1;
-          if (j + 2 < nchunks) raw1 = ldg_nc(col + min(slot + 2 * kChunk, ncol - 1));
-        } else {
-          key = slot < nblk * 64 ? raw0 + (slot & 63) : (slot < nblk * 64 + ncol ? raw0 : -1);
-          if ((unsigned)key >= (unsigned)p.sk) key = -1;
-          raw0 = raw1;
-          if (j + 2 < nchunks) {
-            const int s2 = slot + 2 * kChunk;
-            if (VIS && s2 < nblk * 64 && blk == nullptr) {
-              raw1 = (s2 >> 6) << 6;  // a dense tile: block i starts at key 64 i
-            } else {
-              const int ci = min(max(s2 - nblk * 64, 0), max(ncol - 1, 0));
-              raw1 = ldg_nc(s2 < nblk * 64 ? blk + (s2 >> 6) : col + ci);
+        if (nchunks < 0) break;
+        if (nchunks == 0) continue;
+        const int hkv = h / p.rep;
+        const char* src = reinterpret_cast<const char*>((is_v ? static_cast<const T*>(p.v) + b * p.v_sb + hkv * p.v_sh
+                                                              : static_cast<const T*>(p.k) + b * p.k_sb + hkv * p.k_sh) + c * 8);
+        const int32_t* blk = dense ? nullptr : p.blk_idx + trow * p.blk_stride;  // no table: blocks 0, 64, 128, ...
+        const int32_t* col = p.col_idx + trow * p.col_stride;
+        if (!is_v) {
+          // the Q buffer is free once the last S product of the tile before the previous one has been computed
+          if (!mbar_wait(&bars.qempty[n & 1], ((n >> 1) & 1) ^ 1)) { timed_out = true; break; }
+          const T* qb = static_cast<const T*>(p.q) + b * p.q_sb + h * p.q_sh;
+          unsigned char* qt = q_s + (n & 1) * kQTile;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {  // Q tile: rows beyond the sequence are zero
+            const int pce = pt + i * 128, r = pce >> 4, cq = pce & 15;
+            const bool ok = row0 + r < row_end;
+            cp_async16(smem_addr(qt + tile_off(64, r, cq)), qb + (int64_t)(ok ? row0 + r : 0) * p.q_ss + cq * 8, ok);
+          }
+          cp_async_arrive_noinc(&bars.qfull[n & 1]);
+        }
+        // K and V have producer warps of their own, so neither copy waits behind the other's stage:
+        // a K stage is free as soon as S has been computed from it, a V stage only after the PV
+        // product.  Raw index loads run two chunks ahead and are only interpreted at the top of a
+        // later iteration, so the in-order warp never stalls on them.
+        // a tile without dense blocks (every non-causal tile): slot s is entry s of the column list
+        const bool plain = nblk == 0;
+        for (int j = 0; j < nchunks; ++j, ++g) {
+          const int slot = j * kChunk + my_slot;
+          int key;
+          if (plain) {
+            key = (slot < ncol && (unsigned)raw0 < (unsigned)p.sk) ? raw0 : -1;
+            raw0 = raw1;
+            if (j + 2 < nchunks) raw1 = ldg_nc(col + min(slot + 2 * kChunk, ncol - 1));
+          } else {
+            key = slot < nblk * 64 ? raw0 + (slot & 63) : (slot < nblk * 64 + ncol ? raw0 : -1);
+            if ((unsigned)key >= (unsigned)p.sk) key = -1;
+            raw0 = raw1;
+            if (j + 2 < nchunks) {
+              const int s2 = slot + 2 * kChunk;
+              if (VIS && s2 < nblk * 64 && blk == nullptr) {
+                raw1 = (s2 >> 6) << 6;  // a dense tile: block i starts at key 64 i
+              } else {
+                const int ci = min(max(s2 - nblk * 64, 0), max(ncol - 1, 0));
+                raw1 = ldg_nc(s2 < nblk * 64 ? blk + (s2 >> 6) : col + ci);
+              }
             }
           }
-        }
-        if (!is_v) {
-          keys_s[g & 7][my_slot] = key;
-          // unused slots, and keys that some row of the tile may not see, make the chunk take the masking pass
-          const bool flag = key < 0 || (p.causal && key > p.q_offset + row0);
-          const int any = __any_sync(0xffffffffu, flag);
-          if (lane == 0) mask_s[g & 7][pw] = any;
-        }
-        int keys[16];
-        {
-          int* buf = xk + (g & 1) * 32;
-          buf[lane] = max(key, 0);  // an unused slot copies row 0: its scores are masked and its P is zero
-          __syncwarp();
-          const int4* x4 = reinterpret_cast<const int4*>(buf + (lane & 16));
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int4 q4 = x4[i];
-            keys[4 * i] = q4.x; keys[4 * i + 1] = q4.y; keys[4 * i + 2] = q4.z; keys[4 * i + 3] = q4.w;
+          if (!is_v) {
+            keys_s[g & 7][my_slot] = key;
+            // unused slots, and keys that some row of the tile may not see, make the chunk take the masking pass
+            const bool flag = key < 0 || (p.causal && key > p.q_offset + row0);
+            const int any = __any_sync(0xffffffffu, flag);
+            if (lane == 0) mask_s[g & 7][pw] = any;
           }
-        }
-        uint64_t* full = is_v ? &bars.vfull[stage] : &bars.kfull[stage];
-        if (!mbar_wait(is_v ? &bars.vempty[stage] : &bars.kempty[stage], round ^ 1)) { timed_out = true; break; }
-        const uint32_t dst = smem_addr(is_v ? v_s : k_s) + (uint32_t)stage * kKvTile + dst_off;
+          int keys[16];
+          {
+            int* buf = xk + (g & 1) * 32;
+            buf[lane] = max(key, 0);  // an unused slot copies row 0: its scores are masked and its P is zero
+            __syncwarp();
+            const int4* x4 = reinterpret_cast<const int4*>(buf + (lane & 16));
 #pragma unroll
-        for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * stride);
-        cp_async_arrive_noinc(full);
-        static_assert(kKStages == kVStages, "one ring position for both kinds of producer");
-        if (++stage == kKStages) { stage = 0; round ^= 1; }
+            for (int i = 0; i < 4; ++i) {
+              const int4 q4 = x4[i];
+              keys[4 * i] = q4.x; keys[4 * i + 1] = q4.y; keys[4 * i + 2] = q4.z; keys[4 * i + 3] = q4.w;
+            }
+          }
+          uint64_t* full = is_v ? &bars.vfull[stage] : &bars.kfull[stage];
+          if (!mbar_wait(is_v ? &bars.vempty[stage] : &bars.kempty[stage], round ^ 1)) { timed_out = true; break; }
+          const uint32_t dst = smem_addr(is_v ? v_s : k_s) + (uint32_t)stage * kKvTile + dst_off;
+          const int row_bytes = is_v ? p.v_row_bytes : p.k_row_bytes;
+          if (row_bytes != 0) {  // one 32-bit multiplication into the 64-bit address per row
+#pragma unroll
+            for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * row_bytes);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * ((is_v ? p.v_ss : p.k_ss) * 2));
+          }
+          cp_async_arrive_noinc(full);
+          static_assert(kKStages == kVStages, "one ring position for both kinds of producer");
+          if (++stage == kKStages) { stage = 0; round ^= 1; }
+        }
+        ++n;
       }
-      ++n;
-    }
+    };
+    if (warp < 12) produce(std::false_type{});
+    else produce(std::true_type{});
     cp_async_commit();
     cp_async_wait<0>();  // nothing of this thread may still be in flight when the CTA retires
   } else if (warp >= 16) {
