@@ -25,7 +25,7 @@
 // and the tensor-memory latencies between them; both groups of a scheduler share its special-function unit), then, in the
 // sparse form, the gather beside them.  Measured on one B200 with the former kernel (P in shared memory, eight warps in
 // lockstep on one chunk, 64-row gathered tiles for dense rows): 32 heads x 32 K tokens causal at the reference's default
-// arguments 1.97 -> 1.73 ms for the whole operator; dense causal, 28 query heads on 4 KV heads, 8192 tokens, 0.855 -> 0.504 ms
+// arguments 1.97 -> 1.69 ms for the whole operator (1.75 while the gather multiplied 64-bit row offsets); dense causal, 28 query heads on 4 KV heads, 8192 tokens, 0.855 -> 0.504 ms
 // (560 -> 950 TFLOP/s; 0.519 while the dense form too read a quarter of the scores twice for want of registers).
 #include "va_common.cuh"
 #include "va_sm100.cuh"
@@ -224,11 +224,16 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
         out[4 * i] = q4.x; out[4 * i + 1] = q4.y; out[4 * i + 2] = q4.z; out[4 * i + 3] = q4.w;
       }
     };
-    auto copy_tile = [&](unsigned char* tile_s, const T* base, int64_t stride, const int (&keys)[16], uint64_t* full) {
+    auto copy_tile = [&](unsigned char* tile_s, const T* base, int64_t stride, int row_bytes, const int (&keys)[16], uint64_t* full) {
       const uint32_t dst = smem_addr(tile_s) + dst_off;
-      const T* src = base + c * 8;
+      const char* src = reinterpret_cast<const char*>(base + c * 8);
+      if (row_bytes != 0) {  // one 32-bit multiplication into the 64-bit address per row
 #pragma unroll
-      for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * stride);
+        for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * row_bytes);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * (stride * 2));
+      }
       cp_async_arrive_noinc(full);
     };
     {
@@ -249,11 +254,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
         if (!is_v) {
           const int ks = j % kKStages, ku = j / kKStages;
           if (!mbar_wait(&bars.kempty[ks], (ku & 1) ^ 1)) { timed_out = true; break; }
-          copy_tile(k_s + (size_t)ks * kTileBytes, kb, p.k_ss, keys, &bars.kfull[ks]);
+          copy_tile(k_s + (size_t)ks * kTileBytes, kb, p.k_ss, p.k_row_bytes, keys, &bars.kfull[ks]);
         } else {
           const int vs = j % kVStages, vu = j / kVStages;
           if (!mbar_wait(&bars.vempty[vs], (vu & 1) ^ 1)) { timed_out = true; break; }
-          copy_tile(v_s + (size_t)vs * kTileBytes, vb, p.v_ss, keys, &bars.vfull[vs]);
+          copy_tile(v_s + (size_t)vs * kTileBytes, vb, p.v_ss, p.v_row_bytes, keys, &bars.vfull[vs]);
         }
       }
     }
