@@ -72,3 +72,19 @@ def test_dense_rows(dtype, s, bshd):
     ref = torch.nn.functional.scaled_dot_product_attention(q.float(), k.float().repeat_interleave(3, 1),
                                                            v.float().repeat_interleave(3, 1), is_causal=True)
     _close(out, ref)
+
+
+@pytest.mark.parametrize("pq", [64, 128])
+def test_repeated_rows(pq):
+    """V of one row that is read as many (a stride of 0): its row comes out, whatever the weights."""
+    from vecattention_b200.api import _sparse_attn_bhsd
+    from vecattention_b200.dispatch import Full_prefill
+    g = torch.Generator(device=DEV).manual_seed(9)
+    q, k = (torch.randn(1, 2, 400, 128, generator=g, device=DEV).bfloat16() for _ in range(2))
+    one = torch.randn(1, 2, 1, 128, generator=g, device=DEV).bfloat16()
+    v = one.expand(1, 2, 400, 128)
+    nq = -(-400 // pq)
+    count = torch.full((1, 2, nq), 200, dtype=torch.int32, device=DEV)
+    index = torch.arange(0, 400, 2, dtype=torch.int32, device=DEV).expand(1, 2, nq, 200).contiguous()
+    _close(_sparse_attn_bhsd(q, k, v, pq, None, None, count, index, False), v.float())
+    _close(Full_prefill(q, k, v), v.float())

@@ -512,6 +512,8 @@ int launch_attn128(const AttnParams& p, int dtype, int batch, cudaStream_t strea
 bool launch_dense128(const AttnParams& p, int dtype, int batch, cudaStream_t stream, int* rc) {
   DenseMaps maps;
   const int kv_heads = p.heads / p.rep, bf16 = dtype == VA_BF16;
+  auto forward = [&](int64_t sb, int64_t sh, int64_t ss) { return ss > 0 && (kv_heads == 1 || sh > 0) && (batch == 1 || sb > 0); };
+  if (!forward(p.k_sb, p.k_sh, p.k_ss) || !forward(p.v_sb, p.v_sh, p.v_ss)) return false;  // repeated or reversed rows
   if (!encode_rows_map(&maps.k, bf16, p.k, batch, kv_heads, p.sk, p.k_sb, p.k_sh, p.k_ss, kChunk) ||
       !encode_rows_map(&maps.v, bf16, p.v, batch, kv_heads, p.sk, p.v_sb, p.v_sh, p.v_ss, kChunk))
     return false;
