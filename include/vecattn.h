@@ -123,6 +123,9 @@ int va_select_workspace_bytes(const va_select_args* args, size_t* bytes);
  *   lse        optional (B,H,Sq) float32 contiguous: natural-log sum of exp(score * scale) over the
  *              row's visible keys (the reference API's return_softmax_lse); -inf for a row without keys.
  *   Indices must satisfy 0 <= idx < Sk.
+ * A key that is listed but hidden by the causal rule has weight 0, and its row of v is multiplied by it all
+ * the same (unused places of a tile's last 128 keys stand for row 0 of v): an Inf or NaN there makes rows of
+ * the tile NaN.  In the dense rows below these are the rows of the same 64-key block.
  *
  * Vision-slice composition in one launch (vision_mode = 1; pq 64, causal, Sq == Sk, q_offset 0).
  * Replaces the three attention calls and the concatenation of the "vecattention" branch of

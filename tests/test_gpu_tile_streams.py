@@ -88,3 +88,21 @@ def test_repeated_rows(pq):
     index = torch.arange(0, 400, 2, dtype=torch.int32, device=DEV).expand(1, 2, nq, 200).contiguous()
     _close(_sparse_attn_bhsd(q, k, v, pq, None, None, count, index, False), v.float())
     _close(Full_prefill(q, k, v), v.float())
+
+
+@pytest.mark.parametrize("s,row", [(700, 0), (700, 63), (700, 64), (700, 100), (700, 320), (700, 699), (100, 99)])
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+def test_dense_rows_and_values_that_are_not_finite(s, row, bad):
+    """Keys after a row's own have weight zero, and a row of V that is not finite reaches back no further than its 64-key
+    block, which the operator's tiles take as a whole.  (One batch entry and head has it, the others none.)"""
+    from vecattention_b200.dispatch import Full_prefill
+    g = torch.Generator(device=DEV).manual_seed(row)
+    q = torch.randn(2, 4, s, 128, generator=g, device=DEV).bfloat16()
+    k, v = (torch.randn(2, 2, s, 128, generator=g, device=DEV).bfloat16() for _ in range(2))
+    ref = Full_prefill(q, k, v)
+    v[1, 1, row] = bad
+    out = Full_prefill(q, k, v)
+    before = row // 64 * 64
+    assert torch.equal(out[1, 2:, :before], ref[1, 2:, :before])
+    assert not out[1, 2:, row:].isfinite().any()
+    assert torch.equal(out[0], ref[0]) and torch.equal(out[1, :2], ref[1, :2])

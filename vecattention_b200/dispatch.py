@@ -27,7 +27,8 @@ SPARSITY_RECORD = threading.local()  # .attention_latency_list: [(start event, e
 def Full_prefill(query_states: torch.Tensor, key_states: torch.Tensor, value_states: torch.Tensor, causal: bool = True
                  ) -> torch.Tensor:
     """Dense softmax attention, (B,H,S,D) in and out; causal rows see the keys up to their own position
-    counted from the end of the keys (bottom-right aligned, as the reference's library call is)."""
+    counted from the end of the keys (bottom-right aligned, as the reference's library call is).  Later keys have
+    weight 0; an Inf or NaN in ``value_states`` still reaches the rows of its 64-key block before it (as 0 * Inf)."""
     b, h, sq, _ = query_states.shape
     sk = key_states.shape[2]
     dev = query_states.device
