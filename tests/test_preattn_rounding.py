@@ -1,6 +1,7 @@
 """The rotation of qk_norm_rope rounds the double-precision result once, also where the fp32 arithmetic that serves nearly
 all pairs cannot decide: next to the middle between two 16-bit values, at magnitudes where products over- or underflow,
-at zeros and infinities.  Equality is exact; no tolerance."""
+on both sides of the type's largest value, at zeros and infinities.  All bits are compared, signs of zero included, except
+that any NaN equals any other."""
 import pytest
 import torch
 
@@ -9,7 +10,7 @@ from oracle import vecattn_oracle as O
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("what", ["ordinary", "boundaries", "extremes"])
+@pytest.mark.parametrize("what", ["ordinary", "boundaries", "extremes", "overflow", "zeros"])
 def test_rotation_rounds_once(built_library, dtype, what):
     if not torch.cuda.is_available():
         pytest.fail("GPU tests need a CUDA device")
@@ -35,9 +36,21 @@ def test_rotation_rounds_once(built_library, dtype, what):
         cos = cos * 2.0 ** torch.randint(-50, 30, cos.shape, generator=g)
         sin[::3] = 0.0
         sin[1::5] *= 2.0 ** -50
+    elif what == "overflow":
+        # results within two fp32 places of the middle between the largest value and what would be the next one
+        bits, top = (8, 127) if dtype == torch.bfloat16 else (11, 15)
+        x = (2 - 2.0 ** (1 - bits)) * 2.0 ** top * torch.where(x < 0, -1.0, 1.0)
+        middle = (2 - 2.0 ** -bits) / (2 - 2.0 ** (1 - bits))
+        cos = middle * (1 + torch.randint(-2, 3, cos.shape, generator=g) * 2.0 ** -23)
+        sin[:] = 0.0
+    elif what == "zeros":
+        x = torch.where(x < 0, -0.0, 0.0)
+        x[..., 7::64] = 1.0
+        cos[5::50], sin[7::50] = float("inf"), float("nan")
     x, cos, sin = x.to(dtype), cos.contiguous(), sin.contiguous()
     q, k = qk_norm_rope(x.cuda(), x.cuda(), None, None, 1e-6, cos.cuda(), sin.cuda(), 0, heads=h)
     ref = O.rope_interleaved(x.view(1, s, h, 128).transpose(1, 2), cos, sin)
     for got in (q.cpu(), k.cpu()):
-        assert torch.equal(got.isnan(), ref.isnan())
-        assert torch.equal(got.nan_to_num(0.0), ref.nan_to_num(0.0))
+        number = ~ref.isnan()
+        assert torch.equal(~got.isnan(), number)
+        assert torch.equal(got.contiguous().view(torch.int16)[number], ref.contiguous().view(torch.int16)[number])
