@@ -85,7 +85,9 @@ __device__ __forceinline__ void turn(const float (&y)[8], const float (&c)[4], c
 // memory, which one CTA per row with one piece or two per thread in flight was not (2.4 TB/s).  A CTA holds as many
 // whole rows as fit eight warps.
 constexpr int NP = 4;  // pieces per lane
-template <int DT>
+// ROTATE: the call has tables.  The norm alone is a kernel of its own: with the rotation's registers and branches around it,
+// it took 0.612 ms (0.579 before the rotation was done in fp32), alone 0.521 (40 heads, 75 600 tokens).
+template <int DT, bool ROTATE>
 __global__ void __launch_bounds__(256, 4) qk_norm_rope_rows_kernel(const va_norm_rope_args a, int64_t rows, int W, int rows_per_cta) {
   using T = typename Elem<DT>::T;
   __shared__ float part[8];  // [row of the CTA * W + warp of the row]
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(256, 4) qk_norm_rope_rows_kernel(const va_norm
   const uint64_t rstd2 = pair2(rstd, rstd);
 
   const int rs = s - a.rope_skip;  // row of the cos / sin tables; the first rope_skip tokens are not rotated
-  const bool rotate = live && a.cos != nullptr && rs >= 0;
+  const bool rotate = ROTATE && live && rs >= 0;
   float cc[4] = {}, sv[4] = {};
   if (rotate) {  // a lane's pieces lie 32 W pieces apart, whole heads: all of them sit at the same place of their head
     const int64_t at = (int64_t)rs * (kHeadDim / 2) + (lane & 15) * 4;
@@ -183,7 +185,8 @@ int launch_rows_dt(const va_norm_rope_args& a, cudaStream_t stream) {
   const int W = (pieces + 32 * NP - 1) / (32 * NP);                                 // 1 .. 8 (hidden sizes up to 8192)
   const int per = 8 / W;
   dim3 grid((unsigned)((rows + per - 1) / per), 2, 1);
-  qk_norm_rope_rows_kernel<DT><<<grid, 32 * W * per, 0, stream>>>(a, rows, W, per);
+  auto kern = a.cos ? qk_norm_rope_rows_kernel<DT, true> : qk_norm_rope_rows_kernel<DT, false>;
+  kern<<<grid, 32 * W * per, 0, stream>>>(a, rows, W, per);
   return cudaGetLastError() == cudaSuccess ? VA_OK : VA_ERR_CUDA;
 }
 
