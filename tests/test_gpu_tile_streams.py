@@ -106,3 +106,35 @@ def test_dense_rows_and_values_that_are_not_finite(s, row, bad):
     assert torch.equal(out[1, 2:, :before], ref[1, 2:, :before])
     assert not out[1, 2:, row:].isfinite().any()
     assert torch.equal(out[0], ref[0]) and torch.equal(out[1, :2], ref[1, :2])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("begin,end", [(37, 3300), (0, 3500), (1, 3499), (1000, 1087), (3000, 3300)])
+def test_vision_span_over_many_tiles(dtype, begin, end):
+    """The one-launch composition with several tiles for every SM: sparse and dense tiles and skipped ones (those before
+    the span) follow one another in a CTA.  Dense rows against a plain softmax; all rows the same bits as three launches."""
+    from vecattention_b200 import VecAttention_prefill_vision
+    g = torch.Generator(device=DEV).manual_seed(begin + end)
+    s, h, hkv = 3500, 28, 4
+    q = torch.randn(1, h, s, 128, generator=g, device=DEV).to(dtype)
+    k, v = (torch.randn(1, hkv, s, 128, generator=g, device=DEV).to(dtype) for _ in range(2))
+    one, three = (VecAttention_prefill_vision(q, k, v, 0.8, 64, 16, 16, True, 65536, vision_start_position=begin,
+                                              vision_end_position=end, fused=f) for f in (True, False))
+    assert torch.equal(one, three)
+    ref = torch.nn.functional.scaled_dot_product_attention(q.float(), k.float().repeat_interleave(h // hkv, 1),
+                                                           v.float().repeat_interleave(h // hkv, 1), is_causal=True)
+    for rows in (slice(0, begin), slice(end, s)):
+        if rows.start < rows.stop:
+            _close(one[:, :, rows], ref[:, :, rows])
+
+
+@pytest.mark.parametrize("pq,bk,group", [(64, 16, 16), (128, 128, 1)])
+def test_causal_tiles_head_by_head(pq, bk, group):
+    """Causal calls list the tiles of all heads by length where K and V have at most 64 MB, and head by head above: the
+    same bits both ways.  16 heads of 8700 tokens are 68 MB, four of them 17."""
+    from vecattention_b200 import VecAttention_prefill
+    g = torch.Generator(device=DEV).manual_seed(pq)
+    h, s = 16, 8700
+    q, k, v = (torch.randn(1, h, s, 128, generator=g, device=DEV).bfloat16() for _ in range(3))
+    run = lambda i, n: VecAttention_prefill(*(t[:, i:i + n] for t in (q, k, v)), 0.8, pq, bk, group, True, 16384)  # noqa: E731
+    assert torch.equal(run(0, h), torch.cat([run(i, 4) for i in range(0, h, 4)], dim=1))
