@@ -38,10 +38,8 @@ int sparse_attn(const va_attn_args& a, cudaStream_t stream) {
   if (p.vis_on && p.vis_begin >= p.vis_end) {  // every row is dense: 128-row tiles on streamed K and V take 0.50 ms where
     // gathered 64-row tiles took 0.86 (28 query heads on 4 KV heads, 8192 tokens).  A composition with sparse rows keeps its
     // dense tiles in the 64-row launch: they are few, and a launch of their own would leave most SMs idle.
-    AttnParams d = p;
-    d.vis_begin = d.vis_end = 0;
     int rc;
-    if (launch_dense128(d, a.dtype, a.batch, stream, &rc)) return rc;
+    if (launch_dense128(p, a.dtype, a.batch, stream, &rc)) return rc;
   }
   return a.pq == 64 ? launch_attn64(p, a.dtype, a.batch, stream) : launch_attn128(p, a.dtype, a.batch, stream);
 }

@@ -69,8 +69,8 @@ struct DenseMaps {
   CUtensorMap k, v;
 };
 
-// DENSE: full causal attention of rows [0, vis_begin) and [vis_end, sq) (one sequence for queries and keys): a tile's
-// keys are 0, 1, 2, ... up to its last row, so K and V tiles are contiguous and two threads stream them by TMA.
+// DENSE: full causal attention of all rows (one sequence for queries and keys): a tile's keys are 0, 1, 2, ... up to its
+// last row, so K and V tiles are contiguous and two threads stream them by TMA.
 template <int DT, bool DENSE>
 __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p, const __grid_constant__ DenseMaps maps) {
   using T = typename Elem<DT>::T;
@@ -89,13 +89,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
   place(p, (int)gridDim.x, blockIdx.x, blockIdx.y, tile, h);
   const int b = blockIdx.z;
   const int hkv = h / p.rep;
-  int row0 = tile * PQ, row_end = p.sq;  // rows of the tile at or past row_end do not exist
-  if constexpr (DENSE) {
-    const int n_before = (p.vis_begin + PQ - 1) / PQ;
-    if (tile < n_before) row_end = p.vis_begin;
-    else row0 = p.vis_end + (tile - n_before) * PQ;
-    row_end = min(row_end, row0 + PQ);
-  }
+  const int row0 = tile * PQ, row_end = DENSE ? min(p.sq, row0 + PQ) : p.sq;  // rows at or past row_end do not exist
   const int64_t trow = DENSE ? 0 : ((int64_t)b * p.heads + h) * p.nq + tile;
   const int nblk = !DENSE && p.blk_count ? __ldg(p.blk_count + trow) : 0;
   const int ncol = DENSE ? row_end : __ldg(p.col_count + trow);
@@ -190,53 +184,52 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
           for (int i = max(0, j - stages); i < j; ++i) mbar_wait(&full[i % stages], (i / stages) & 1);
       }
     } else {
-    // Copy geometry.  A warp covers two key rows per instruction: lanes 0-15 the sixteen 16-byte
-    // pieces of row rbase + 8 i, lanes 16-31 those of the next row.  Because the rows of one thread
-    // differ by multiples of 8, its swizzled piece position is the same in all of them and the
-    // shared-memory destinations are one base address plus i * 1024.
-    // Each lane fetches ONE key index per chunk (that of row rbase + 8 * (lane & 15)), two chunks
-    // ahead; the sixteen indices a thread needs are then exchanged through shared memory.
-    const int pw = (pt >> 5), hi = lane >> 4, c = lane & 15;
-    const int rbase = 2 * pw + hi;
-    const uint32_t dst_off = tile_off(128, rbase, c);
-    const int my_slot = rbase + 8 * c;
-    auto fetch_raw = [&](int j) -> int {
-      const int slot = j * kChunk + my_slot;
-      const int ci = min(max(slot - nblk * 64, 0), max(ncol - 1, 0));
-      return ldg_nc(slot < nblk * 64 ? blk + (slot >> 6) : col + ci);
-    };
-    auto decode = [&](int j, int raw) -> int {
-      const int slot = j * kChunk + my_slot;
-      const int key = slot < nblk * 64 ? raw + (slot & 63) : (slot < nslots ? raw : -1);
-      return (key >= 0 && key < p.sk) ? key : -1;
-    };
-    // through a small exchange array of the warp: one store and four 16-byte loads per thread instead of sixteen
-    // shuffles; two buffers, so the next chunk's stores cannot overtake this chunk's loads
-    int* xk = xk_s[warp - 8][0];
-    auto spread = [&](int j, int key, int (&out)[16]) {
-      int* buf = xk + (j & 1) * 32;
-      buf[lane] = max(key, 0);  // an unused slot copies row 0: its scores are masked and its P is zero
-      __syncwarp();
-      const int4* src = reinterpret_cast<const int4*>(buf + (lane & 16));
+      // Copy geometry.  A warp covers two key rows per instruction: lanes 0-15 the sixteen 16-byte
+      // pieces of row rbase + 8 i, lanes 16-31 those of the next row.  Because the rows of one thread
+      // differ by multiples of 8, its swizzled piece position is the same in all of them and the
+      // shared-memory destinations are one base address plus i * 1024.
+      // Each lane fetches ONE key index per chunk (that of row rbase + 8 * (lane & 15)), two chunks
+      // ahead; the sixteen indices a thread needs are then exchanged through shared memory.
+      const int pw = (pt >> 5), hi = lane >> 4, c = lane & 15;
+      const int rbase = 2 * pw + hi;
+      const uint32_t dst_off = tile_off(128, rbase, c);
+      const int my_slot = rbase + 8 * c;
+      auto fetch_raw = [&](int j) -> int {
+        const int slot = j * kChunk + my_slot;
+        const int ci = min(max(slot - nblk * 64, 0), max(ncol - 1, 0));
+        return ldg_nc(slot < nblk * 64 ? blk + (slot >> 6) : col + ci);
+      };
+      auto decode = [&](int j, int raw) -> int {
+        const int slot = j * kChunk + my_slot;
+        const int key = slot < nblk * 64 ? raw + (slot & 63) : (slot < nslots ? raw : -1);
+        return (key >= 0 && key < p.sk) ? key : -1;
+      };
+      // through a small exchange array of the warp: one store and four 16-byte loads per thread instead of sixteen
+      // shuffles; two buffers, so the next chunk's stores cannot overtake this chunk's loads
+      int* xk = xk_s[warp - 8][0];
+      auto spread = [&](int j, int key, int (&out)[16]) {
+        int* buf = xk + (j & 1) * 32;
+        buf[lane] = max(key, 0);  // an unused slot copies row 0: its scores are masked and its P is zero
+        __syncwarp();
+        const int4* src = reinterpret_cast<const int4*>(buf + (lane & 16));
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int4 q4 = src[i];
-        out[4 * i] = q4.x; out[4 * i + 1] = q4.y; out[4 * i + 2] = q4.z; out[4 * i + 3] = q4.w;
-      }
-    };
-    auto copy_tile = [&](unsigned char* tile_s, const T* base, int64_t stride, int row_bytes, const int (&keys)[16], uint64_t* full) {
-      const uint32_t dst = smem_addr(tile_s) + dst_off;
-      const char* src = reinterpret_cast<const char*>(base + c * 8);
-      if (row_bytes != 0) {  // one 32-bit multiplication into the 64-bit address per row
+        for (int i = 0; i < 4; ++i) {
+          const int4 q4 = src[i];
+          out[4 * i] = q4.x; out[4 * i + 1] = q4.y; out[4 * i + 2] = q4.z; out[4 * i + 3] = q4.w;
+        }
+      };
+      auto copy_tile = [&](unsigned char* tile_s, const T* base, int64_t stride, int row_bytes, const int (&keys)[16], uint64_t* full) {
+        const uint32_t dst = smem_addr(tile_s) + dst_off;
+        const char* src = reinterpret_cast<const char*>(base + c * 8);
+        if (row_bytes != 0) {  // one 32-bit multiplication into the 64-bit address per row
 #pragma unroll
-        for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * row_bytes);
-      } else {
+          for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * row_bytes);
+        } else {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * (stride * 2));
-      }
-      cp_async_arrive_noinc(full);
-    };
-    {
+          for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * (stride * 2));
+        }
+        cp_async_arrive_noinc(full);
+      };
       int keys[16];
       int raw0 = fetch_raw(0), raw1 = nchunks > 1 ? fetch_raw(1) : 0;
       for (int j = 0; j < nchunks && !timed_out; ++j) {
@@ -261,7 +254,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
           copy_tile(v_s + (size_t)vs * kTileBytes, vb, p.v_ss, p.v_row_bytes, keys, &bars.vfull[vs]);
         }
       }
-    }
     }
     cp_async_commit();
     cp_async_wait<0>();  // nothing of this thread may still be in flight when the CTA retires
@@ -538,7 +530,7 @@ bool launch_dense128(const AttnParams& p, int dtype, int batch, cudaStream_t str
   if (!encode_rows_map(&maps.k, bf16, p.k, batch, kv_heads, p.sk, p.k_sb, p.k_sh, p.k_ss, kChunk) ||
       !encode_rows_map(&maps.v, bf16, p.v, batch, kv_heads, p.sk, p.v_sb, p.v_sh, p.v_ss, kChunk))
     return false;
-  const int tiles = (p.vis_begin + 127) / 128 + (p.sq - p.vis_end + 127) / 128;
+  const int tiles = (p.sq + 127) / 128;
   *rc = bf16 ? launch<VA_BF16, true>(p, maps, tiles, batch, stream) : launch<VA_FP16, true>(p, maps, tiles, batch, stream);
   return true;
 }
