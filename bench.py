@@ -34,13 +34,12 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
-# dram__bytes_read.sum + dram__bytes_write.sum per launch of the attention kernel, from the ncu
-# capture summarised under profiles/ (workload -> bytes); None until a capture exists
-# workload -> bytes; c4 was captured at full size (one-pass metrics): profiles/launch_list_c4.md
-NCU_TRAFFIC_BYTES = {"c2h8": 303.4e6, "c4": 6.30e9 + 0.725e9}  # profiles/sparse_attn64_kernel_c2h8.md
-NCU_SELECT_TRAFFIC_BYTES = {"c4": (729.9e6 + 12.9e6) + (810.9e6 + 658.3e6) + (670.5e6 + 1.71e9)}  # pool + mask + expand
+# workload -> dram__bytes_read.sum + dram__bytes_write.sum of a launch, from the one-pass ncu captures summarised in
+# profiles/launch_list_c4.md (c4 at full size) and profiles/sparse_attn64_kernel_c2h8.md
+NCU_TRAFFIC_BYTES = {"c2h8": 299.1e6, "c4": 7.65e9 + 0.726e9}
+NCU_SELECT_TRAFFIC_BYTES = {"c4": (729.9e6 + 13.3e6) + (824.5e6 + 658.4e6) + (670.2e6 + 1.71e9)}  # pool + mask + expand
 # the capture is of 8 heads; DRAM traffic of this kernel grows in proportion to the heads processed
-NCU_TRAFFIC_PER_HEAD_32K = 303.4e6 / 8
+NCU_TRAFFIC_PER_HEAD_32K = 299.1e6 / 8
 D = 128
 CONFIG_HEADS = {"c2": 32, "c3": 40, "c4": 24, "c5": 28, "c2h8": 8}
 
@@ -332,11 +331,11 @@ def _rooflines(wl, peaks, stage, flops, counts):
     full = wl.heads == CONFIG_HEADS.get(wl.name)
     traffic = (NCU_TRAFFIC_PER_HEAD_32K * wl.heads if wl.name in ("c2", "c2h8") else
                NCU_TRAFFIC_BYTES.get(wl.name) if full else None)
-    roofline = {"kernel": "sparse_attn64_kernel" if wl.q_pooling_size == 64 else "sparse_attn128_kernel", "bound": "tensor",
+    roofline = {"kernel": "sparse_attn64_kernel" if wl.q_pooling_size == 64 else "attn128_kernel", "bound": "tensor",
                 "achieved": achieved_tf, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
                 "frac": achieved_tf / peaks["bf16_tflops"], "traffic": traffic,
                 "traffic_note": ("ncu capture of 8 heads x 32 K tokens, scaled by heads" if wl.name in ("c2", "c2h8") else
-                                 "one-pass ncu capture of this workload at full size (profiles/launch_list_c4.md): 1.5x the "
+                                 "one-pass ncu capture of this workload at full size (profiles/launch_list_c4.md): 1.8x the "
                                  "algorithmic 4.6 GB, K/V of two 61 MB heads do not both stay in the 126 MB L2" if traffic else
                                  "not captured for this workload or head count"),
                 "peak_source": peaks["_source"] + " burst"}

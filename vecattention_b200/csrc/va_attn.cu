@@ -32,8 +32,9 @@ int sparse_attn(const va_attn_args& a, cudaStream_t stream) {
   p.scale_log2 = scale * 1.4426950408889634f;
   // One head after another keeps a head's K and V in L2 while its tiles run; where those of all heads fit half of it,
   // the tiles of all heads are listed by length instead, so that no head's longest tiles start last: 28 query heads on 4 KV
-  // heads, 9001 tokens (18 MB) 0.403 -> 0.370 ms, 20011 tokens with a vision span (41 MB) 1.02 -> 0.87 ms; 64 K tokens (134 MB)
-  // stay head by head, at 6.3 ms.
+  // heads, 9001 tokens (18 MB) 0.403 -> 0.370 ms, 20011 tokens with a vision span (41 MB) 1.02 -> 0.87 ms.  The line is not where
+  // the two meet: listed by length, whole calls with 64 / 96 / 128 / 256 MB of K and V run 1.08-1.17 / 1.09-1.14 / 1.05-1.13 /
+  // 1.04-1.13 times as fast with 64-row tiles, 1.00-1.04 times with 128-row ones (16 to 32 heads, 8 K to 64 K tokens).
   p.by_length = a.causal && (int64_t)a.batch * a.kv_heads * a.sk * kHeadDim * 2 * 2 <= (64 << 20);
   if (p.vis_on && p.vis_begin >= p.vis_end) {  // every row is dense: 128-row tiles on streamed K and V take 0.50 ms where
     // gathered 64-row tiles took 0.86 (28 query heads on 4 KV heads, 8192 tokens).  A composition with sparse rows keeps its

@@ -29,7 +29,7 @@ __device__ __forceinline__ typename Elem<DT>::T from_double(double x) {
 // ---- the rotation of a pair, rounded once ----
 // x = a c - b s rounded once to the 16-bit type is what the double-precision expression gives.  Its conversions and the
 // rounding from double cost the kernel, which is bound by issue slots, more than the norm did, so nearly all pairs are
-// done in fp32 with the same result (40 heads, 75 600 tokens: 0.995 -> 0.827 ms, 3.15 -> 3.8 TB/s; a branch per pair instead of
+// done in fp32 with the same result (40 heads, 75 600 tokens: 0.995 -> 0.82 ms, 3.15 -> 3.8 TB/s; a branch per pair instead of
 // one per piece of four: 0.886):
 //  * Kahan's product sum (w = b s; f = a c - w; t = f + (w - b s), both fma exact to their last rounding) is within
 //    1.5 units in the last place of x (Jeannerod, Louvet, Muller, "Further analysis of Kahan's algorithm for the accurate

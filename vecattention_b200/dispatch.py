@@ -6,8 +6,9 @@ device time as a pair of CUDA events on a thread-local list, and optionally dump
 threshold tuner.  The reference's other methods (xattn, flex, anchor) are separate baselines and
 raise ``NotImplementedError`` here.
 
-Dense attention ("full") runs on the vector-sparse kernel with block tables that list every
-64-key block a tile may see; the reference calls flashinfer there (spattn/src/Fullprefill.py).
+Dense attention ("full"): causal with as many keys as queries runs on 128-row tiles that stream K and V (where their strides
+suit a tensor map); otherwise it is the vector-sparse kernel's dense 64-key blocks, from block tables that list every block
+a tile may see.  The reference calls flashinfer there (spattn/src/Fullprefill.py).
 """
 from __future__ import annotations
 
@@ -36,7 +37,7 @@ def Full_prefill(query_states: torch.Tensor, key_states: torch.Tensor, value_sta
     q_off = sk - sq if causal else 0
     if causal and q_off < 0:
         raise VecAttentionArgumentError("causal dense attention needs at least as many keys as queries")
-    if causal and q_off == 0:  # every tile is a table-free dense tile of the kernel's vision-slice mode
+    if causal and q_off == 0:  # vision-slice mode without a sparse row: no table is read
         none = torch.zeros(b, h, nq, dtype=torch.int32, device=dev)
         return _sparse_attn_bhsd(query_states, key_states, value_states, 64, None, None, none,
                                  torch.zeros(b, h, nq, 4, dtype=torch.int32, device=dev), True, vision=(sq, sq))
