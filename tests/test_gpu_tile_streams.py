@@ -130,11 +130,25 @@ def test_vision_span_over_many_tiles(dtype, begin, end):
 
 @pytest.mark.parametrize("pq,bk,group", [(64, 16, 16), (128, 128, 1)])
 def test_causal_tiles_head_by_head(pq, bk, group):
-    """Causal calls list the tiles of all heads by length where K and V have at most 64 MB, and head by head above: the
-    same bits both ways.  16 heads of 8700 tokens are 68 MB, four of them 17."""
+    """Heads whose K and V have at most 64 MB together are listed together, tile by tile: the same bits in any grouping.
+    16 heads of 8700 tokens are 68 MB (two groups of eight), four of them 17 (one group)."""
     from vecattention_b200 import VecAttention_prefill
     g = torch.Generator(device=DEV).manual_seed(pq)
     h, s = 16, 8700
     q, k, v = (torch.randn(1, h, s, 128, generator=g, device=DEV).bfloat16() for _ in range(3))
     run = lambda i, n: VecAttention_prefill(*(t[:, i:i + n] for t in (q, k, v)), 0.8, pq, bk, group, True, 16384)  # noqa: E731
     assert torch.equal(run(0, h), torch.cat([run(i, 4) for i in range(0, h, 4)], dim=1))
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("heads,kv,s", [(5, 5, 45000), (6, 3, 45001), (3, 3, 140000)])
+def test_groups_of_heads(heads, kv, s, causal):
+    """Groups of unequal size (5 KV heads of 23 MB: 2 + 2 + 1), of several query heads per KV head, and of one head because
+    its K and V alone exceed 64 MB: the same bits as a call per KV head."""
+    from vecattention_b200 import VecAttention_prefill
+    g = torch.Generator(device=DEV).manual_seed(s)
+    q = torch.randn(1, heads, s, 128, generator=g, device=DEV, dtype=torch.bfloat16)
+    k, v = (torch.randn(1, kv, s, 128, generator=g, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    rep = heads // kv
+    run = lambda i, n: VecAttention_prefill(q[:, i * rep:(i + n) * rep], k[:, i:i + n], v[:, i:i + n], 0.97, 64, 16, 16, causal, 32768)  # noqa: E731
+    assert torch.equal(run(0, kv), torch.cat([run(i, 1) for i in range(kv)], dim=1))

@@ -30,12 +30,16 @@ int sparse_attn(const va_attn_args& a, cudaStream_t stream) {
   p.causal = a.causal; p.q_offset = a.q_offset;
   const float scale = a.softmax_scale > 0.f ? a.softmax_scale : 0.08838834764831845f;
   p.scale_log2 = scale * 1.4426950408889634f;
-  // One head after another keeps a head's K and V in L2 while its tiles run; where those of all heads fit half of it,
-  // the tiles of all heads are listed by length instead, so that no head's longest tiles start last: 28 query heads on 4 KV
-  // heads, 9001 tokens (18 MB) 0.403 -> 0.370 ms, 20011 tokens with a vision span (41 MB) 1.02 -> 0.87 ms.  The line is not where
-  // the two meet: listed by length, whole calls with 64 / 96 / 128 / 256 MB of K and V run 1.08-1.17 / 1.09-1.14 / 1.05-1.13 /
-  // 1.04-1.13 times as fast with 64-row tiles, 1.00-1.04 times with 128-row ones (16 to 32 heads, 8 K to 64 K tokens).
-  p.by_length = a.causal && (int64_t)a.batch * a.kv_heads * a.sk * kHeadDim * 2 * 2 <= (64 << 20);
+  // Heads whose K and V together fit half of L2 are listed together, tile by tile: no head's longest causal tiles start
+  // last, and the SMs gather from several heads at a time.  Whole calls, head by head and so, with the K and V of one group:
+  // 28 query heads on 4 KV heads, causal, 9001 tokens (all heads, 18 MB) 389 -> 350 us, 20011 with a vision span (41 MB) 984 -> 854,
+  // 64 K (2 KV heads, 64 MB) 6069 -> 5912; 32 heads, 48 K, causal (2, 48 MB) 4290 -> 4096; not causal, 8 heads x 16 000 (33 MB)
+  // 320 -> 286, 32 x 32 K (3, 50 MB) 3299 -> 3235.  Groups of up to 100 MB are slower where the keys are spread over the
+  // sequence: 32 x 32 K 3383, 16 x 100 K not causal 14 002 -> 14 833; of up to 24 MB: 3291 and 4280.
+  const int64_t kv_bytes = (int64_t)a.sk * kHeadDim * 2 * 2;
+  const int64_t fit = kv_bytes < (64 << 20) ? (64 << 20) / kv_bytes : 1;
+  const int groups = (int)((a.kv_heads + fit - 1) / fit);
+  p.group = (a.kv_heads + groups - 1) / groups * p.rep;
   if (p.vis_on && p.vis_begin >= p.vis_end) {  // every row is dense: 128-row tiles on streamed K and V take 0.50 ms where
     // gathered 64-row tiles took 0.86 (28 query heads on 4 KV heads, 8192 tokens).  A composition with sparse rows keeps its
     // dense tiles in the 64-row launch: they are few, and a launch of their own would leave most SMs idle.

@@ -27,19 +27,16 @@ struct AttnParams {
   // from tiles that need no tables, rows [vis_begin, vis_end) the sparse attention of their tile; `nq` then counts
   // the table tiles (rows [0, vis_end)) and the grid has the dense tiles behind them.
   int vis_on, vis_begin, vis_end;
-  int by_length;  // causal: the grid lists the longest tile of every head, then every head's second longest, ...
+  int group;  // heads whose tiles are listed together: tile 0 of each of them, then tile 1 of each, ...
 };
 
-// The tile and head of CTA (x, y) of a grid of (tiles, heads).  Causal tiles grow with their index; the longest are
-// started first, so that the grid's tail is made of short ones.
+// The tile and head of CTA (x, y) of a grid of (tiles, heads): one group of heads after another.  Causal tiles grow with
+// their index; the longest are started first, so that a group's tail is made of short ones.
 __device__ __forceinline__ void place(const AttnParams& p, int tiles, uint32_t x, uint32_t y, int& tile, int& head) {
-  if (p.by_length) {
-    const uint32_t at = y * (uint32_t)tiles + x;
-    head = (int)(at % (uint32_t)p.heads);
-    x = at / (uint32_t)p.heads;
-  } else {
-    head = (int)y;
-  }
+  const uint32_t at = y * (uint32_t)tiles + x, first = at / ((uint32_t)tiles * p.group) * p.group;  // the group's first head
+  const uint32_t in_group = at - first * tiles, n = min((uint32_t)p.group, p.heads - first);       // (the last group may be smaller)
+  head = (int)(first + in_group % n);
+  x = in_group / n;
   tile = p.causal ? tiles - 1 - (int)x : (int)x;
 }
 
