@@ -8,22 +8,30 @@
 //    share one KV head form one row list (row R -> head hkv*rep + R/nq, tile R%nq); a CTA owns 128
 //    consecutive rows of that list and walks the keys of its KV head once, 128 keys per tile, in
 //    ascending order, so the running (prefix) maximum of a key-block group is a per-thread register.
-//    Warp roles (608 threads, one CTA per SM):
-//      warps 0-15  row walkers, by turns: warp w can reach TMEM lane quarter w % 4 (32 pooled rows) and takes
-//                 every fourth key tile (tiles n with n % 4 == w / 4, accumulator buffer w / 4), so the four
-//                 warps of a scheduler work on four different tiles.  A thread walks its row's whole tile:
-//                 it reads the 128 estimates and forms the maxima of the tile's key blocks, receives the
+//    Warp roles (352 threads, one CTA per SM):
+//      warps 0-7  row walkers, by turns: warp w can reach TMEM lane quarter w % 4 (32 pooled rows) and takes
+//                 every other key tile (tiles n with n % 2 == w / 4), so the two
+//                 warps of a scheduler work on different tiles.  A thread walks its row's whole tile:
+//                 it takes the 128 estimates into registers, which frees the accumulator buffer, and forms the maxima of the
+//                 tile's key blocks, receives the
 //                 row's running maximum after the previous tile from the warp that walked it (one float
 //                 per row through shared memory, an mbarrier per warp pair), forms the running maximum
-//                 entering every block and hands the one after its tile on at once; then it reads the
-//                 estimates again, builds the 128 keep bits fp32(s + gap) >= m and stores them as one
-//                 16-byte piece of the row's mask.  With few row blocks the key range is cut into up to
+//                 entering every block and hands the one after its tile on at once; then it
+//                 builds the 128 keep bits fp32(s + gap) >= m and stores them as one
+//                 16-byte piece of the row's mask.  Where every tile is a whole number of key-block groups nothing is
+//                 handed on.  With few row blocks the key range is cut into up to
 //                 four segments (one CTA each): a CTA still walks from the first tile for the maxima but
 //                 writes keep bits only for its own segment.
-//      warp 16    one thread streams K: a TMA tensor-map copy per 128-key tile (two boxes of 128 rows
+//      warp 8     one thread streams K: a TMA tensor-map copy per 128-key tile (two boxes of 128 rows
 //                 x 128 bytes, 128-byte swizzle) into a 4-stage ring; rows past the sequence read as zeros.
-//      warps 17,18 one thread each issues S_t = Q~ K_t^T for alternate tiles, 128 x 128 x 128 as eight
+//      warps 9,10 one thread each issues S_t = Q~ K_t^T for alternate tiles, 128 x 128 x 128 as eight
 //                 tcgen05.mma, into one of four 128-column accumulator buffers in tensor memory.
+//    What bounds it: the walkers' instructions, some 500 a tile and scheduler beside 518 clk of tensor arithmetic, of which the
+//    ALU takes two clk each (64 three-input maxima, 64 byte permutes and logic operations).  A tile takes about 1060 clk.
+//    Sixteen warps that read their estimates from tensor memory twice, 96 registers each, spilled; launches then and now:
+//    k_local_size 128 (32 heads x 32 K, causal) 210 -> 122 us; 16: 32 heads x 32 K 168 -> 153, 28/4 heads x 64 K causal 316 -> 286,
+//    9001 tokens, groups of one block, 48 -> 42.  (A funnel shift per estimate in place of conversion, permute and
+//    logic: 1-3 % slower.)
 //    All hand-offs are mbarriers with bounded waits; a timeout sets VA_STATUS_TIMEOUT.
 //
 // 2. select_expand_kernel: one warp per pooled row turns the row's keep bits into its ascending
@@ -53,6 +61,7 @@ struct SelectParams {
   int wpad;           // words per mask row (whole groups of four key tiles)
   int heads, kv_heads, rep, nq, sk;
   int pq, group_k_block;
+  uint32_t starts;    // see WalkArgs
   int nseg;           // CTAs per block of 128 rows, each writing the keep bits of one segment of the key range
   int by_length;      // causal, whole row blocks per head: blockIdx.x lists the row blocks of all heads longest walk first
   int tail_from, tail_seg;  // tail_seg > 0: a flat grid; the CTAs from number tail_from on (the last, partial wave of
@@ -67,13 +76,14 @@ constexpr int kTile = 128;   // keys per tile
 constexpr int kTileBytes = 128 * 256;
 constexpr int kStages = 4;   // K ring
 constexpr int kSBufs = 4;    // accumulator buffers in tensor memory (4 x 128 columns = all of it)
-constexpr int kThreads = 608;  // 16 walker warps, the K producer, two MMA issuers
-constexpr int kWalkerWarps = 16;
+constexpr int kTurns = 2;      // walker warps of a lane quarter, which take key tiles by turns
+constexpr int kWalkerWarps = 4 * kTurns;
+constexpr int kThreads = 32 * (kWalkerWarps + 3);  // the walkers, the K producer, two MMA issuers
 constexpr size_t kSmem = 1024 + (size_t)kTileBytes * (1 + kStages);
 
 struct Barriers {
   uint64_t kfull[kStages], kempty[kStages], sfull[kSBufs], sempty[kSBufs];
-  uint64_t hand[4][4];  // [lane quarter][turn]: that warp has published the rows' running maximum after its tile
+  uint64_t hand[4][kTurns];  // [lane quarter][turn]: that warp has published the rows' running maximum after its tile
 };
 
 // End (exclusive) of the keys pooled row `tile` of the chunk may select, spattn/src/kernels/
@@ -129,15 +139,13 @@ __device__ __forceinline__ void unpack2(uint64_t x, uint32_t& lo, uint32_t& hi) 
 }
 
 // ---- the row walkers ------------------------------------------------------------------------------
-// Sixteen warps; warp (qtr, turn) = (w % 4, w / 4) owns the pooled rows of TMEM lane quarter qtr (a warp
-// reaches only the quarter w % 4) on every fourth key tile, n = turn (mod 4), which lives in accumulator
-// buffer `turn`.  A thread handles its row's whole tile: first the maxima of the tile's key blocks
-// (independent of earlier tiles), then, once the warp of the previous tile has handed over the rows'
+// Eight warps; warp (qtr, turn) = (w % 4, w / 4) owns the pooled rows of TMEM lane quarter qtr (a warp
+// reaches only the quarter w % 4) on every other key tile.  A thread handles its row's whole tile: first the maxima of the
+// tile's key blocks (independent of earlier tiles), then, once the warp of the previous tile has handed over the rows'
 // running maximum, the running maximum entering every block, which it hands on at once, and last the
-// keep bits of the 128 keys, read from tensor memory a second time.  The four warps of a quarter sit on one
-// scheduler and are in different phases of different tiles, so one's latencies hide behind another's work.
+// keep bits of the 128 keys, from the estimates it still holds.
 struct WalkShared {
-  float rmx[4][4][32];  // [lane quarter][turn][lane]: running maximum after that warp's latest tile
+  float rmx[4][kTurns][32];  // [lane quarter][turn][lane]: running maximum after that warp's latest tile
 };
 
 // what a walker thread knows about its CTA and its row
@@ -148,6 +156,7 @@ struct WalkArgs {
   int lo, k_hi;        // key range the CTA walks
   int sk, hi;          // sequence length; end of this thread's row
   int G;               // key blocks per group
+  uint32_t starts;     // groups inside a tile: bit k is set if block k of a tile starts one
   float gap;
   uint32_t* mrow;      // this thread's mask row
 };
@@ -160,91 +169,102 @@ __device__ __forceinline__ bool wait_fast(uint64_t* bar, uint32_t parity) {
 
 // Keep bits of 32 estimates: fp32(s + gap) >= m  <=>  fp32(s + gap) - m is not negative (the difference of
 // two floats has the exact sign).  m_lo applies to estimates 0..15, m_hi to 16..31.  Two packed additions per
-// pair of estimates and one funnel shift per estimate that moves the sign bit into a byte of the mask, last key
-// first; four independent chains of eight shifts, joined by byte permutes, so key c ends up in bit c.
+// pair of estimates.  A difference keeps its sign when it is converted to a 16-bit float, two in one instruction; a byte
+// permute turns the signs of keys g, 8 + g, 16 + g and 24 + g into four bytes of zeros or ones, and one logic
+// operation files bit g of each of them: key c ends up in bit c.
 __device__ __forceinline__ uint32_t keep_bits(const uint32_t (&v)[32], uint64_t gap2, float m_lo, float m_hi) {
-  uint32_t neg[4];
+  const uint64_t nm2[2] = {pack2(-m_lo, -m_lo), pack2(-m_hi, -m_hi)};
+  uint32_t neg = 0u;
 #pragma unroll
-  for (int q = 3; q >= 0; --q) {
-    const float m = q >= 2 ? m_hi : m_lo;
-    const uint64_t nm2 = pack2(-m, -m);
-    uint32_t x = 0u;
+  for (int g = 0; g < 8; g += 2) {
+    uint32_t d[2][4];
 #pragma unroll
-    for (int c = q * 8 + 7; c > q * 8; c -= 2) {
-      uint32_t d_lo, d_hi;
-      unpack2(add2(add2(pack2u(v[c - 1], v[c]), gap2), nm2), d_lo, d_hi);
-      x = __funnelshift_l(d_hi, x, 1);
-      x = __funnelshift_l(d_lo, x, 1);
+    for (int q = 0; q < 4; ++q)
+      unpack2(add2(add2(pack2u(v[q * 8 + g], v[q * 8 + g + 1]), gap2), nm2[q >> 1]), d[0][q], d[1][q]);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      uint32_t a, b, spread;
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(a) : "f"(__uint_as_float(d[e][1])), "f"(__uint_as_float(d[e][0])));
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(b) : "f"(__uint_as_float(d[e][3])), "f"(__uint_as_float(d[e][2])));
+      asm("prmt.b32 %0, %1, %2, 0xfdb9;" : "=r"(spread) : "r"(a), "r"(b));  // bytes 1 and 3 of both, the sign eight times
+      neg |= spread & (0x01010101u << (g + e));
     }
-    neg[q] = x;  // eight sign bits in the low byte
   }
-  const uint32_t lo16 = __byte_perm(neg[0], neg[1], 0x0040), hi16 = __byte_perm(neg[2], neg[3], 0x0040);
-  return ~__byte_perm(lo16, hi16, 0x5410);
+  return ~neg;
 }
 
-// Walk every fourth key tile of the CTA for the rows of lane quarter `qtr`.  Returns false if a wait ran
-// out.  BK = k_local_size; ALIGNED: groups of key blocks begin only where tiles begin.
-template <int BK, bool ALIGNED>
+// Where groups of key blocks begin.
+enum Groups {
+  kAnywhere,  // any block of a tile
+  kAtTiles,   // only at a tile's first block (a group is a whole number of tiles)
+  kInTiles,   // at every tile's first block, and perhaps inside it (a tile is a whole number of groups): tiles are independent
+};
+
+// Walk every kTurns-th key tile of the CTA for the rows of lane quarter `qtr`.  Returns false if a wait ran
+// out.  BK = k_local_size.
+template <int BK, Groups GROUPS>
 __device__ __forceinline__ bool walk_rows(const WalkArgs& a, Barriers& bars, WalkShared& sh, int qtr, int turn, int lane) {
   constexpr int NBT = kTile / BK;  // key blocks per tile
-  const uint32_t taddr = a.tmem + ((uint32_t)(qtr * 32) << 16) + (uint32_t)turn * 128;
+  const uint32_t taddr0 = a.tmem + ((uint32_t)(qtr * 32) << 16);
   const uint64_t gap2 = pack2(a.gap, a.gap);
-  uint64_t* const sfull = &bars.sfull[turn];
-  uint64_t* const sempty = &bars.sempty[turn];
-  uint64_t* const hand_in = &bars.hand[qtr][(turn + 3) & 3];
+  const int before = (turn + kTurns - 1) % kTurns;  // the turn that has the tile before this warp's
+  uint64_t* const hand_in = &bars.hand[qtr][before];
   uint64_t* const hand_out = &bars.hand[qtr][turn];
-  const float* rm_in = &sh.rmx[qtr][(turn + 3) & 3][lane];
+  const float* rm_in = &sh.rmx[qtr][before][lane];
   float* rm_out = &sh.rmx[qtr][turn][lane];
   const int ntiles = a.t_hi - a.t_lo;
-  const unsigned tpg = ALIGNED ? (unsigned)(((int64_t)a.G * BK) / kTile) : 1u;  // tiles per group of key blocks
+  const unsigned tpg = GROUPS == kAtTiles ? (unsigned)(((int64_t)a.G * BK) / kTile) : 1u;  // tiles per group of key blocks
+  unsigned tg = GROUPS == kAtTiles ? (unsigned)(a.t_lo + turn) % tpg : 0u;                 // the tile's place in its group
+  const uint32_t starts = GROUPS == kInTiles ? a.starts : 1u;  // blocks of a tile with which a group starts
   const int t_in_lo = (a.lo + kTile - 1) / kTile;  // first tile wholly at or after lo
   const int t_in_hi = min(a.k_hi, a.sk) / kTile;   // tiles before this one end at or before k_hi
 
-  for (int n = turn; n < ntiles; n += 4) {
-    const int t = a.t_lo + n, key_t = t * kTile;
-    const uint32_t par = (uint32_t)(n >> 2) & 1u;
-    const bool inner = ALIGNED && t >= t_in_lo && t < t_in_hi;  // no range tests, no group start inside the tile
-    if (!wait_fast(sfull, par)) return false;
+  for (int n = turn; n < ntiles; n += kTurns) {
+    const int t = a.t_lo + n, key_t = t * kTile, sb = n % kSBufs;
+    const bool inner = GROUPS != kAnywhere && t >= t_in_lo && t < t_in_hi;  // no range tests
+    if (!wait_fast(&bars.sfull[sb], (uint32_t)(n / kSBufs) & 1u)) return false;
     tc_fence_after();
+    // ---- the row's 128 estimates; the accumulator buffer is free again ----
+    uint32_t v[4][32];
+#pragma unroll
+    for (int c4 = 0; c4 < 4; ++c4) tmem_ld32(taddr0 + (uint32_t)(sb * 128 + c4 * 32), v[c4]);
+    tmem_wait_ld();
+    tc_fence_before();
+    mbar_arrive(&bars.sempty[sb]);
     // ---- maxima of the tile's key blocks (keys past the sequence end never count) ----
     float pm[NBT];
+    if (inner || key_t + kTile <= a.sk) {
 #pragma unroll
-    for (int k = 0; k < NBT; ++k) pm[k] = -INFINITY;
-#pragma unroll
-    for (int c4 = 0; c4 < 4; ++c4) {
-      uint32_t v[32];
-      tmem_ld32(taddr + c4 * 32, v);
-      tmem_wait_ld();
-      if (key_t + c4 * 32 + 32 <= a.sk) {
-        if (BK == 16) {
-          pm[(2 * c4) % NBT] = max_of<16>(v);
-          pm[(2 * c4 + 1) % NBT] = max_of<16>(v + 16);
+      for (int k = 0; k < NBT; ++k) {
+        if constexpr (BK == 16) {
+          pm[k] = max_of<16>(v[k / 2] + (k & 1) * 16);
         } else {
-          const int k = (c4 * 32 / BK) % NBT;
-          pm[k] = fmaxf(pm[k], max_of<32>(v));
-        }
-      } else {
+          pm[k] = max_of<32>(v[k * (BK / 32)]);
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (key_t + c4 * 32 + j < a.sk) {
-            const int k = ((c4 * 32 + j) / BK) % NBT;
-            pm[k] = fmaxf(pm[k], __uint_as_float(v[j]));
-          }
+          for (int i = 1; i < BK / 32; ++i) pm[k] = fmaxf(pm[k], max_of<32>(v[k * (BK / 32) + i]));
+        }
       }
+    } else {
+#pragma unroll
+      for (int k = 0; k < NBT; ++k) pm[k] = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < kTile; ++j)
+        if (key_t + j < a.sk) pm[j / BK] = fmaxf(pm[j / BK], __uint_as_float(v[j / 32][j % 32]));
     }
     // ---- the rows' running maximum after the previous tile, from the warp that walked it ----
     float run = -INFINITY;
-    if (n > 0) {
-      if (!wait_fast(hand_in, (uint32_t)((n - 1) >> 2) & 1u)) return false;
+    if (GROUPS != kInTiles && n > 0) {
+      if (!wait_fast(hand_in, (uint32_t)((n - 1) / kTurns) & 1u)) return false;
       run = *rm_in;
     }
     // ---- running maximum entering / after every block; handed on before the keep bits are formed ----
     float rm[NBT];
     uint32_t on_bits = 0xffffffffu;  // bit k: block k lies inside the walked key range
     if (inner) {
-      if ((unsigned)t % tpg == 0u) run = -INFINITY;  // a new group of key blocks starts with this tile
+      if (tg == 0u) run = -INFINITY;  // a new group of key blocks starts with this tile
 #pragma unroll
       for (int k = 0; k < NBT; ++k) {
+        if (GROUPS == kInTiles && k > 0 && (starts >> k & 1u)) run = -INFINITY;
         run = fmaxf(run, pm[k]);
         rm[k] = run;
       }
@@ -263,43 +283,41 @@ __device__ __forceinline__ bool walk_rows(const WalkArgs& a, Barriers& bars, Wal
         rm[k] = run;
       }
     }
-    *rm_out = run;
-    mbar_arrive(hand_out);
-    if (t < a.t_keep) {  // another CTA writes this tile's keep bits: only the running maximum was needed
-      tc_fence_before();
-      mbar_arrive(sempty);
-      continue;
+    if (GROUPS != kInTiles) {
+      *rm_out = run;
+      mbar_arrive(hand_out);
     }
+    if (GROUPS == kAtTiles) {
+      tg += kTurns;
+      while (tg >= tpg) tg -= tpg;
+    }
+    if (t < a.t_keep) continue;  // another CTA writes this tile's keep bits: only the running maximum was needed
     // ---- keep bits of the 128 keys ----
     uint32_t w[4];
 #pragma unroll
-    for (int c4 = 0; c4 < 4; ++c4) {
-      uint32_t v[32];
-      tmem_ld32(taddr + c4 * 32, v);
-      tmem_wait_ld();
-      if (c4 == 3) {  // the accumulator buffer is free again
-        tc_fence_before();
-        mbar_arrive(sempty);
+    for (int c4 = 0; c4 < 4; ++c4)
+      w[c4] = keep_bits(v[c4], gap2, rm[c4 * 32 / BK], rm[(c4 * 32 + 16) / BK]);
+    if (!inner) {
+#pragma unroll
+      for (int c4 = 0; c4 < 4; ++c4) {
+        if (!((on_bits >> (c4 * 32 / BK)) & 1u)) w[c4] &= 0xffff0000u;
+        if (!((on_bits >> ((c4 * 32 + 16) / BK)) & 1u)) w[c4] &= 0x0000ffffu;
       }
-      const int k_lo = BK == 16 ? 2 * c4 : (c4 * 32 / BK) % NBT, k_hi16 = BK == 16 ? 2 * c4 + 1 : k_lo;
-      uint32_t m = keep_bits(v, gap2, rm[k_lo % NBT], rm[k_hi16 % NBT]);
-      if (!inner) {
-        if (!((on_bits >> (k_lo % NBT)) & 1u)) m &= 0xffff0000u;
-        if (!((on_bits >> (k_hi16 % NBT)) & 1u)) m &= 0x0000ffffu;
+    }
+    if (key_t + kTile > a.hi) {  // keys at or past the row's limit are cut off
+#pragma unroll
+      for (int c4 = 0; c4 < 4; ++c4) {
+        const int room = a.hi - (key_t + c4 * 32);
+        if (room < 32) w[c4] = room <= 0 ? 0u : (w[c4] & ((1u << room) - 1u));
       }
-      const int room = a.hi - (key_t + c4 * 32);  // keys at or past the row's limit are cut off
-      if (room < 32) m = room <= 0 ? 0u : (m & ((1u << room) - 1u));
-      w[c4] = m;
     }
     *reinterpret_cast<uint4*>(a.mrow + (size_t)t * 4) = make_uint4(w[0], w[1], w[2], w[3]);
   }
   return true;
 }
 
-// BK = k_local_size.  ALIGNED: a key-block group (group_k_block * BK keys) is a whole number of
-// tiles, so groups begin only where tiles begin and a tile inside the walked key range needs no
-// per-block bookkeeping.
-template <int DT, int BK, bool ALIGNED>
+// BK = k_local_size.
+template <int DT, int BK, Groups GROUPS>
 __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_constant__ CUtensorMap kmap, const SelectParams p) {
   using T = typename Elem<DT>::T;
   extern __shared__ unsigned char smem_raw[];
@@ -342,7 +360,7 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
     b = cta / (nb * p.kv_heads);
   }
 
-  // ---- per-row limits: walker threads (warps 0-15) own row (warp % 4) * 32 + lane ----
+  // ---- per-row limits: walker threads own row (warp % 4) * 32 + lane ----
   const bool is_walker = warp < kWalkerWarps;
   const int wrow = (warp & 3) * 32 + lane;
   const int R = row_base + wrow;
@@ -407,12 +425,12 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
     }
     for (int s = 0; s < kSBufs; ++s) {
       mbar_init(&bars.sfull[s], 1);
-      mbar_init(&bars.sempty[s], 4 * 32);  // the four warps (one per lane quarter) that walk the buffer's tiles
+      mbar_init(&bars.sempty[s], 4 * 32);  // four warps, one per lane quarter, read a tile
     }
-    for (int s = 0; s < 16; ++s) mbar_init(&bars.hand[s >> 2][s & 3], 32);
+    for (int s = 0; s < 4 * kTurns; ++s) mbar_init(&bars.hand[s / kTurns][s % kTurns], 32);
     fence_proxy_async();
   }
-  if (warp == 17) {
+  if (warp == kWalkerWarps + 1) {
     tmem_alloc(&tmem_base_s, 512);
     tmem_relinquish();
   }
@@ -422,7 +440,7 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
   const uint32_t tmem = tmem_base_s;
   bool timed_out = false;
 
-  if (warp == 16) {
+  if (warp == kWalkerWarps) {
     // ======================= K tile producer (one thread, TMA) =======================
     if (lane == 0) {
       int issued = 0, s = 0;
@@ -441,17 +459,17 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
         for (int n = max(0, issued - kStages); n < issued; ++n) mbar_wait(&bars.kfull[n % kStages], (n / kStages) & 1);
       }
     }
-  } else if (warp >= 17) {
+  } else if (warp > kWalkerWarps) {
     // ======================= MMA issuers =======================
-    // Two threads (warps 17 and 18) take alternate tiles: while one is held by the tensor pipe's queue, the
+    // Two threads take alternate tiles: while one is held by the tensor pipe's queue, the
     // other has already passed the barrier waits of the next tile, so the pipe never runs dry between tiles.
     if (lane == 0) {
       constexpr uint32_t in16 = DT == VA_BF16 ? 1u : 0u;
       constexpr uint32_t idesc = umma_idesc(128, 128, in16, 0, 0);
       const uint64_t qd = umma_desc(smem_addr(q_s), 16, 1024), kd0 = umma_desc(smem_addr(k_s), 16, 1024);
-      int s = warp - 17, sb = warp - 17;
+      int s = warp - kWalkerWarps - 1, sb = s;
       uint32_t kpar = 0, spar = 1;  // phase parities of the stage's "full" and the buffer's "empty" barrier
-      for (int t = t_lo + (warp - 17); t < t_hi; t += 2) {
+      for (int t = t_lo + s; t < t_hi; t += 2) {
         if (!wait_fast(&bars.kfull[s], kpar) || !wait_fast(&bars.sempty[sb], spar)) { timed_out = true; break; }
         tc_fence_after();
         umma_k128_rows128(tmem + (uint32_t)sb * 128, qd, kd0 + (uint64_t)(s * (kTileBytes >> 4)), idesc);
@@ -473,14 +491,15 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
     a.sk = p.sk;
     a.hi = hi;
     a.G = p.group_k_block;
+    a.starts = p.starts;
     a.gap = p.gaps ? __ldg(p.gaps + b * p.gaps_sb + h) : p.gap;
     a.mrow = p.mask + ((size_t)(b * p.kv_heads + hkv) * p.rows_pad + row_base + wrow) * p.wpad;
-    timed_out = !walk_rows<BK, ALIGNED>(a, bars, wsh, warp & 3, warp >> 2, lane);
+    timed_out = !walk_rows<BK, GROUPS>(a, bars, wsh, warp & 3, warp >> 2, lane);
   }
   if (timed_out && p.status) atomicOr(p.status, VA_STATUS_TIMEOUT);
   tc_fence_before();
   __syncthreads();
-  if (warp == 17) tmem_dealloc(tmem, 512);
+  if (warp == kWalkerWarps + 1) tmem_dealloc(tmem, 512);
 }
 
 // ---- keep bits -> ascending index lists ---------------------------------------------------------
@@ -582,8 +601,10 @@ __global__ void __launch_bounds__(kExpandWarps * 32) select_expand_kernel(const 
 
 template <int DT, int BK>
 int launch_bk(const SelectParams& p, const CUtensorMap& kmap, int batch, cudaStream_t stream) {
-  const bool aligned = ((int64_t)p.group_k_block * BK) % kTile == 0;
-  auto kern = aligned ? select_mask_kernel<DT, BK, true> : select_mask_kernel<DT, BK, false>;
+  const int64_t group = (int64_t)p.group_k_block * BK;
+  auto kern = select_mask_kernel<DT, BK, kAnywhere>;
+  if (kTile % group == 0) kern = select_mask_kernel<DT, BK, kInTiles>;
+  else if (group % kTile == 0) kern = select_mask_kernel<DT, BK, kAtTiles>;
   // per-device attribute; setting it on every launch keeps multi-device processes correct
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess) return VA_ERR_CUDA;
   dim3 grid(p.rows_pad / kRows * p.nseg, p.kv_heads, batch);
@@ -643,6 +664,8 @@ int select(const va_select_args& a, cudaStream_t stream) {
   p.sk = a.sk;
   p.pq = a.pq;
   p.group_k_block = a.group_k_block;
+  p.starts = 0;
+  for (int k = 0; k < 8; k += a.group_k_block < 8 ? a.group_k_block : 8) p.starts |= 1u << k;
   p.causal = a.causal;
   p.wo_initial = a.wo_initial;
   p.compat_bsq = a.compat_bsq;
