@@ -152,3 +152,39 @@ def test_groups_of_heads(heads, kv, s, causal):
     rep = heads // kv
     run = lambda i, n: VecAttention_prefill(q[:, i * rep:(i + n) * rep], k[:, i:i + n], v[:, i:i + n], 0.97, 64, 16, 16, causal, 32768)  # noqa: E731
     assert torch.equal(run(0, kv), torch.cat([run(i, 1) for i in range(kv)], dim=1))
+
+
+@pytest.mark.parametrize("heads,kv,s,pq,bk,group,causal", [
+    (4, 4, 2048, 64, 16, 16, False),    # segments of one group each
+    (3, 3, 700, 64, 16, 1, True),       # fewer tiles than segments
+    (14, 2, 9001, 64, 16, 1, True),     # groups inside a tile; row blocks of several heads
+    (14, 2, 9001, 64, 16, 3, True),     # a group starts with a tile every third tile only
+    (5, 5, 12800, 64, 32, 5, False),    # ... every fifth
+    (14, 2, 20011, 64, 16, 100, True),  # ... every 25th, longer than some segments
+    (28, 4, 9001, 64, 16, 8192, True),  # one group: segments walk all keys before them
+    (3, 3, 30000, 64, 16, 8192, False),
+    (40, 20, 5000, 64, 64, 2, False),   # whole waves and a cut rest
+    (4, 4, 9000, 128, 128, 1, True),
+    (4, 2, 9000, 128, 64, 4, True),
+])
+@pytest.mark.parametrize("chunk_tiles", [0, 24])
+def test_selection_in_segments(heads, kv, s, pq, bk, group, causal, chunk_tiles):
+    """The work of a selection is cut into row blocks and key segments by the number of both: the same lists as one query
+    head at a time with 64 tiles a call, which cuts it elsewhere (and, causal, orders the rows differently)."""
+    from vecattention_b200.api import average_vector, fuse_qk_softmax_minp_wo_causal
+    g = torch.Generator(device=DEV).manual_seed(s + group)
+    q = average_vector(torch.randn(1, heads, s, 128, generator=g, device=DEV).bfloat16() + 0.5, pq)
+    k = torch.randn(1, kv, s, 128, generator=g, device=DEV).bfloat16()
+    gap = torch.rand(heads, generator=g, device=DEV) * 0.1 + 0.1
+
+    def lists(q, k, offset, gap):
+        count, index = fuse_qk_softmax_minp_wo_causal(q, k, offset, gap, causal, pq, bk, causal, group, trim=False, chunk_tiles=chunk_tiles)
+        return index.masked_fill_(torch.arange(index.shape[-1], device=DEV) >= count[..., None], -1)
+
+    whole = lists(q, k, 0, gap)
+    step = chunk_tiles or 64
+    for h in range(heads):
+        kh = h // (heads // kv)
+        for t in range(0, q.shape[2], step):
+            part = lists(q[:, h:h + 1, t:t + step], k[:, kh:kh + 1], t, gap[h:h + 1])
+            assert torch.equal(part, whole[:, h:h + 1, t:t + step])

@@ -5,8 +5,8 @@
 //
 // 1. select_mask_kernel: estimate, running maximum and keep test; its result is one keep BIT per
 //    (pooled row, key), written row-major to scratch memory.  The pooled rows of all query heads that
-//    share one KV head form one row list (row R -> head hkv*rep + R/nq, tile R%nq); a CTA owns 128
-//    consecutive rows of that list and walks the keys of its KV head once, 128 keys per tile, in
+//    share one KV head form one row list (row R -> head hkv*rep + R%rep, tile R/rep, so that neighbours see about as many
+//    keys under the causal rule); a CTA owns 128 consecutive rows of that list and walks the keys of its KV head once, 128 keys per tile, in
 //    ascending order, so the running (prefix) maximum of a key-block group is a per-thread register.
 //    Warp roles (352 threads, one CTA per SM):
 //      warps 0-7  row walkers, by turns: warp w can reach TMEM lane quarter w % 4 (32 pooled rows) and takes
@@ -19,9 +19,9 @@
 //                 entering every block and hands the one after its tile on at once; then it
 //                 builds the 128 keep bits fp32(s + gap) >= m and stores them as one
 //                 16-byte piece of the row's mask.  Where every tile is a whole number of key-block groups nothing is
-//                 handed on.  With few row blocks the key range is cut into up to
-//                 four segments (one CTA each): a CTA still walks from the first tile for the maxima but
-//                 writes keep bits only for its own segment.
+//                 handed on.  The key range is cut into segments, one CTA each, where that lets the SMs finish
+//                 together (make_plan): a CTA starts its walk where the group of key blocks starts that its segment begins in,
+//                 for the maxima, and writes keep bits only for its own segment.
 //      warp 8     one thread streams K: a TMA tensor-map copy per 128-key tile (two boxes of 128 rows
 //                 x 128 bytes, 128-byte swizzle) into a 4-stage ring; rows past the sequence read as zeros.
 //      warps 9,10 one thread each issues S_t = Q~ K_t^T for alternate tiles, 128 x 128 x 128 as eight
@@ -47,6 +47,20 @@ namespace va {
 
 using namespace sm100;
 
+// How a launch's work is cut into CTAs.  A CTA has one block of 128 pooled rows and one segment of its keys: tiles
+// [cut[s], cut[s + 1]) from the walk's first tile on.  CTAs below `whole` have all keys of their block; the others are listed in
+// runs of one segment each, run r being CTAs whole + start[r] and up.
+constexpr int kMaxSegments = 32;
+struct Plan {
+  int whole, runs, segments, ctas;
+  int heads;   // KV heads of all batch entries
+  int period;  // tiles after which a group of key blocks starts with a tile again
+  int cut[kMaxSegments + 1];
+  // not causal: run s has segment s of the blocks from number `whole` on.  Causal: run s has segment s of the blocks that fill it,
+  // run segments + s that of the blocks that end inside it, so that the longest walks come first; top: the last block of a run.
+  int start[2 * kMaxSegments], top[2 * kMaxSegments];
+};
+
 struct SelectParams {
   const void* avg_q;  // (B,H,nq,D)
   const float* gaps;
@@ -62,10 +76,7 @@ struct SelectParams {
   int heads, kv_heads, rep, nq, sk;
   int pq, group_k_block;
   uint32_t starts;    // see WalkArgs
-  int nseg;           // CTAs per block of 128 rows, each writing the keep bits of one segment of the key range
-  int by_length;      // causal, whole row blocks per head: blockIdx.x lists the row blocks of all heads longest walk first
-  int tail_from, tail_seg;  // tail_seg > 0: a flat grid; the CTAs from number tail_from on (the last, partial wave of
-                            // equally long walks) are cut into tail_seg key segments each
+  Plan plan;
   int causal, wo_initial, compat_bsq, tile_offset, chunk_tiles;
 };
 
@@ -327,47 +338,37 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
   __shared__ WalkShared wsh;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int hkv = blockIdx.y;
-  int b = blockIdx.z;
   const int nrows = p.rep * p.nq;
-  // causal rows walk more keys the later their tile: the longest walks are started first
-  int bx = p.causal ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
-  if (p.by_length) {
-    // one grid row for all KV heads: CTAs are handed out in blockIdx.x order, so all heads' last 128 tiles come
-    // first, then all heads' last but one, ...: a longest-first schedule over the whole launch
-    const int blocks_per_head = p.nq / kRows, per_rank = p.rep * p.kv_heads;
-    const int rank = (int)blockIdx.x / per_rank, r2 = (int)blockIdx.x % per_rank;
-    hkv = r2 % p.kv_heads;
-    bx = (r2 / p.kv_heads) * blocks_per_head + (blocks_per_head - 1 - rank);
+  // ---- this CTA's row block and segment ----
+  const int blocks = p.rows_pad / kRows;
+  int at = (int)blockIdx.x, seg_from = 0, seg_to = 0x7fffffff, run = 0;
+  if (at >= p.plan.whole) {
+    at -= p.plan.whole;
+    while (run + 1 < p.plan.runs && at >= p.plan.start[run + 1]) ++run;
+    at -= p.plan.start[run];
+    const int s = run < p.plan.segments ? run : run - p.plan.segments;
+    seg_from = p.plan.cut[s];
+    seg_to = p.plan.cut[s + 1];
+    if (!p.causal) at += p.plan.whole;
   }
-  int nseg = p.nseg;
-  int row_base = (bx / p.nseg) * kRows, seg = bx % p.nseg;
-  if (p.tail_seg > 0) {
-    // Equally long walks fill whole waves of SMs except for the last CTAs; those are cut into key segments so that
-    // the last wave is shorter (a segment's CTA re-walks the maxima of the segments before it, the cheap half).
-    const int lin = (int)blockIdx.x, nb = p.rows_pad / kRows;
-    int cta = lin;
-    seg = 0;
-    nseg = 1;
-    if (lin >= p.tail_from) {
-      const int r = lin - p.tail_from;
-      cta = p.tail_from + r / p.tail_seg;
-      seg = r % p.tail_seg;
-      nseg = p.tail_seg;
-    }
-    row_base = (cta % nb) * kRows;
-    hkv = (cta / nb) % p.kv_heads;
-    b = cta / (nb * p.kv_heads);
+  int bx, head_at;  // row block; KV head and batch entry
+  if (p.causal) {   // the later the rows the longer the walk
+    bx = p.plan.top[run] - at / p.plan.heads;
+    head_at = at % p.plan.heads;
+  } else {          // the row blocks of a head side by side: they walk the same keys
+    bx = at % blocks;
+    head_at = at / blocks;
   }
+  const int row_base = bx * kRows, hkv = head_at % p.kv_heads, b = head_at / p.kv_heads;
 
   // ---- per-row limits: walker threads own row (warp % 4) * 32 + lane ----
   const bool is_walker = warp < kWalkerWarps;
   const int wrow = (warp & 3) * 32 + lane;
   const int R = row_base + wrow;
   const bool row_ok = is_walker && R < nrows;
-  const int h = hkv * p.rep + (row_ok ? R / p.nq : 0);
+  const int h = hkv * p.rep + (row_ok ? R % p.rep : 0);
   const int lo = p.wo_initial ? p.pq : 0;
-  const int hi = row_ok ? row_key_limit(p, R % p.nq, BK) : 0;
+  const int hi = row_ok ? row_key_limit(p, R / p.rep, BK) : 0;
 
   if (tid == 0) s_khi = 0;
   __syncthreads();
@@ -379,18 +380,14 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
   }
   __syncthreads();
   const int k_hi = s_khi;                       // CTA-wide end of the key walk
-  const int t_lo = lo / kTile;
+  int t_lo = lo / kTile;
   int t_hi = (k_hi + kTile - 1) / kTile;  // exclusive
-  if (t_lo >= t_hi || k_hi <= lo) return;  // nothing selectable for any row of this CTA (the expansion writes zero counts)
-  // With few row blocks the key range is cut into segments, one CTA each: a CTA walks from the first tile (the
-  // running maximum is a prefix quantity) but forms keep bits only for its own segment, and stops after it.
-  int t_keep = t_lo;
-  if (nseg > 1) {
-    const int per = (t_hi - t_lo + nseg - 1) / nseg;
-    t_keep = t_lo + seg * per;
-    if (t_keep >= t_hi) return;
-    t_hi = min(t_hi, t_keep + per);
-  }
+  // The CTA writes the keep bits of its segment only.  The running maximum is that of a group of key blocks up to here, so
+  // the walk starts where the segment's first group does.
+  const int t_keep = t_lo + seg_from;
+  if (seg_to < t_hi - t_lo) t_hi = t_lo + seg_to;
+  if (k_hi <= lo || t_keep >= t_hi) return;  // nothing selectable here (the expansion writes the counts)
+  t_lo = max(t_lo, t_keep / p.plan.period * p.plan.period);
 
   unsigned char* smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
   unsigned char* q_s = smem;
@@ -405,7 +402,7 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
       const int RR = row_base + r;
       uint4 w = make_uint4(0, 0, 0, 0);
       if (RR < nrows) {
-        const int hh = hkv * p.rep + RR / p.nq, tt = RR % p.nq;
+        const int hh = hkv * p.rep + RR % p.rep, tt = RR / p.rep;
         w = __ldg(reinterpret_cast<const uint4*>(aq + (((int64_t)b * p.heads + hh) * p.nq + tt) * kHeadDim + c * 8));
         uint32_t* ww = reinterpret_cast<uint32_t*>(&w);
 #pragma unroll
@@ -533,7 +530,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32) select_expand_kernel(const 
   const int64_t bh = row / p.nq;
   const int h = (int)(bh % p.heads), b = (int)(bh / p.heads);
   const int hkv = h / p.rep;
-  const int R = (h % p.rep) * p.nq + tile;
+  const int R = tile * p.rep + h % p.rep;
   const int lo = p.wo_initial ? p.pq : 0;
   const int hi = row_key_limit(p, tile, BK);
   const uint32_t* mrow = p.mask + ((size_t)(b * p.kv_heads + hkv) * p.rows_pad + R) * p.wpad;
@@ -607,14 +604,10 @@ int launch_bk(const SelectParams& p, const CUtensorMap& kmap, int batch, cudaStr
   else if (group % kTile == 0) kern = select_mask_kernel<DT, BK, kAtTiles>;
   // per-device attribute; setting it on every launch keeps multi-device processes correct
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess) return VA_ERR_CUDA;
-  dim3 grid(p.rows_pad / kRows * p.nseg, p.kv_heads, batch);
-  if (p.by_length) grid = dim3(p.rows_pad / kRows * p.kv_heads, 1, batch);
-  if (p.tail_seg > 0) {
-    const int ctas = p.rows_pad / kRows * p.kv_heads * batch;
-    grid = dim3(p.tail_from + (ctas - p.tail_from) * p.tail_seg, 1, 1);
+  if (p.plan.ctas > 0) {
+    kern<<<p.plan.ctas, kThreads, kSmem, stream>>>(kmap, p);
+    if (cudaGetLastError() != cudaSuccess) return VA_ERR_CUDA;
   }
-  kern<<<grid, kThreads, kSmem, stream>>>(kmap, p);
-  if (cudaGetLastError() != cudaSuccess) return VA_ERR_CUDA;
   const int64_t total_rows = (int64_t)batch * p.heads * p.nq;
   select_expand_kernel<BK><<<(unsigned)((total_rows + kExpandWarps - 1) / kExpandWarps), kExpandWarps * 32, 0, stream>>>(p, total_rows);
   return cudaGetLastError() == cudaSuccess ? VA_OK : VA_ERR_CUDA;
@@ -647,6 +640,135 @@ size_t select_workspace_bytes(int batch, int heads, int kv_heads, int nq, int sk
   return (size_t)batch * kv_heads * rows_pad * wpad * 4;
 }
 
+// Cut the work into CTAs so that the SMs finish together: the number of segments per row block is the one with the least
+// estimated time, in tiles.  A tile that only feeds the running maximum costs kFeed of one with keep bits, a CTA kSetUp tiles
+// (it loads its rows, fills and drains its pipeline: 3 us).
+static void make_plan(SelectParams& p, int batch, int bk) {
+  constexpr double kFeed = 0.55, kSetUp = 5.0;
+  Plan& pl = p.plan;
+  int sms = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int blocks = p.rows_pad / kRows, t0 = (p.wo_initial ? p.pq : 0) / kTile;
+  const int all = (p.sk + kTile - 1) / kTile;
+  pl.heads = p.kv_heads * batch;
+  const int64_t group = (int64_t)p.group_k_block * bk;  // a divisor or a multiple of the tile, or anything
+  int64_t common = group, rest = kTile;                 // greatest common divisor
+  while (rest) {
+    const int64_t r = common % rest;
+    common = rest;
+    rest = r;
+  }
+  pl.period = (int)(group / common < all ? group / common : all);
+  // tiles walked by a row block: all, or under the causal rule those before its last row's own
+  auto length = [&](int block) {
+    int64_t end = p.sk;
+    if (p.causal) {
+      const int last = (block + 1) * kRows < p.rep * p.nq ? (block + 1) * kRows - 1 : p.rep * p.nq - 1;
+      const int64_t before = ((int64_t)p.tile_offset + last / p.rep) * p.pq;
+      end = before < end ? before : end;
+    }
+    const int n = (int)((end + kTile - 1) / kTile) - t0;
+    return n > 0 ? n : 0;
+  };
+  const int longest = length(blocks - 1);
+  const int64_t ctas = (int64_t)blocks * pl.heads;
+  // segment s of a block that is cut into n: equal ones where a group starts every few tiles; else each is shorter than the
+  // one before by what it walks again, so that all take the same time
+  auto set_cuts = [&](int n) {
+    const int step = (longest + n - 1) / n, whole = (step + pl.period - 1) / pl.period * pl.period;
+    pl.segments = n;
+    pl.cut[0] = 0;
+    if (4 * (whole - step) <= step) {
+      for (int s = 1; s <= n; ++s) pl.cut[s] = (int64_t)s * whole < longest ? s * whole : longest;
+    } else {
+      double left = 1.0, at = 0.0;
+      for (int s = 0; s < n; ++s) left *= 1.0 - kFeed;
+      const double first = longest * kFeed / (1.0 - left);
+      for (int s = 1; s <= n; ++s) {
+        at += first - kFeed * at;
+        pl.cut[s] = (int)(at + 0.999);
+        if (pl.cut[s] > longest) pl.cut[s] = longest;
+      }
+    }
+    pl.cut[n] = longest;
+    while (pl.segments > 1 && pl.cut[pl.segments - 1] >= longest) --pl.segments;
+  };
+  auto segment_cost = [&](int s, int tiles) {  // of a block with that many tiles
+    const int to = tiles < pl.cut[s + 1] ? tiles : pl.cut[s + 1], again = (t0 + pl.cut[s]) % pl.period;
+    return to - pl.cut[s] + kFeed * (again < pl.cut[s] ? again : pl.cut[s]) + kSetUp;
+  };
+  auto cost = [&](int64_t first_block) {  // of the segments as they are cut, first_block: in the order of the heads' blocks
+    double most = 0.0, sum = 0.0;
+    int64_t n = 0;
+    if (!p.causal) {
+      for (int s = 0; s < pl.segments; ++s) {
+        const double c = segment_cost(s, longest);
+        most = c > most ? c : most;
+      }
+      n = (ctas - first_block) * pl.segments;
+      return (double)((n + sms - 1) / sms) * most;
+    }
+    int64_t filled = 0;
+    for (int i = 0; i < blocks; ++i) {
+      const int tiles = length(i);
+      for (int s = 0; s < pl.segments && pl.cut[s] < tiles; ++s, n += pl.heads) {
+        const double c = segment_cost(s, tiles);
+        most = c > most ? c : most;
+        sum += c * pl.heads;
+        if (tiles >= pl.cut[s + 1]) filled += pl.heads;
+      }
+    }
+    // the segments that are filled come first, the others fill the gaps
+    const double waves = (double)((filled + sms - 1) / sms) * most, spread = sum / sms + 0.2 * most;
+    return n <= sms ? most : waves > spread ? waves : spread;
+  };
+  static const int kTry[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 16, 24, 32};
+  int best = 1;
+  int64_t best_whole = 0;
+  double least = 0.0;
+  for (const int n : kTry) {
+    if (n > 1 && (n > longest || ctas >= 8 * (int64_t)sms)) break;
+    set_cuts(n);
+    const double c = cost(0);
+    if (n == 1 || c < 0.97 * least) {
+      least = c;
+      best = n;
+    }
+    const int64_t full = ctas / sms * sms;
+    if (!p.causal && full > 0 && full < ctas) {  // whole waves of uncut blocks, and the rest cut
+      const double w = (double)(full / sms) * (longest + kSetUp) + cost(full);
+      if (w < 0.97 * least) {
+        least = w;
+        best = n;
+        best_whole = full;
+      }
+    }
+  }
+  set_cuts(best);
+  pl.whole = (int)best_whole;
+  int n = 0;
+  pl.runs = 0;
+  auto run_of = [&](int count, int top) {
+    pl.start[pl.runs] = n;
+    pl.top[pl.runs++] = top;
+    n += count * (p.causal ? pl.heads : 1);
+  };
+  if (!p.causal) {
+    for (int s = 0; s < pl.segments; ++s) run_of((int)(ctas - best_whole), 0);
+  } else {
+    int reach[kMaxSegments], fill[kMaxSegments];  // the first block that reaches into segment s, and the first that fills it
+    for (int s = 0, i = 0, j = 0; s < pl.segments; ++s) {
+      while (i < blocks && length(i) <= pl.cut[s]) ++i;
+      while (j < blocks && length(j) < pl.cut[s + 1]) ++j;
+      reach[s] = i;
+      fill[s] = j;
+      run_of(blocks - j, blocks - 1);
+    }
+    for (int s = 0; s < pl.segments; ++s) run_of(fill[s] - reach[s], fill[s] - 1);
+  }
+  pl.ctas = pl.whole + n;
+}
+
 int select(const va_select_args& a, cudaStream_t stream) {
   SelectParams p;
   p.avg_q = a.avg_q;
@@ -672,28 +794,7 @@ int select(const va_select_args& a, cudaStream_t stream) {
   p.tile_offset = a.tile_offset;
   p.chunk_tiles = a.chunk_tiles;
   mask_geometry(a.heads, a.kv_heads, a.nq, a.sk, p.rows_pad, p.wpad);
-  {  // few CTAs: cut the key range so that more SMs take part (each extra segment re-walks the earlier ones' maxima)
-    int sms = 148, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t ctas = (int64_t)(p.rows_pad / kRows) * a.kv_heads * a.batch;
-    const int tiles = (a.sk + kTile - 1) / kTile;
-    int nseg = (int)(sms / (ctas > 0 ? ctas : 1));
-    nseg = nseg < 1 ? 1 : (nseg > 4 ? 4 : nseg);
-    if (tiles < 64 * nseg) nseg = 1;  // short walks gain nothing
-    p.nseg = nseg;
-  }
-  p.by_length = (a.causal && p.nseg == 1 && a.nq % kRows == 0) ? 1 : 0;
-  p.tail_from = p.tail_seg = 0;
-  if (!a.causal && p.nseg == 1) {  // equally long walks: shorten the last, partial wave
-    int sms = 148, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t ctas = (int64_t)(p.rows_pad / kRows) * a.kv_heads * a.batch;
-    const int64_t full = ctas / sms * sms, rest = ctas - full;
-    if (full > 0 && rest > 0 && rest * 2 <= sms && (a.sk + kTile - 1) / kTile >= 128 && ctas < (1 << 30)) {
-      p.tail_from = (int)full;
-      p.tail_seg = (int)(sms / rest < 4 ? sms / rest : 4);
-    }
-  }
+  make_plan(p, a.batch, a.bk);
   if (!a.workspace) return VA_ERR_NULL;
   if (a.workspace_bytes < select_workspace_bytes(a.batch, a.heads, a.kv_heads, a.nq, a.sk)) return VA_ERR_CAPACITY;
   if ((reinterpret_cast<uintptr_t>(a.workspace) & 15u) != 0) return VA_ERR_ALIGN;
