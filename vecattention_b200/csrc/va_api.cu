@@ -7,7 +7,7 @@ namespace va {
 int pool_q(const va_pool_args& a, cudaStream_t stream);
 int select(const va_select_args& a, cudaStream_t stream);
 size_t select_workspace_bytes(int batch, int heads, int kv_heads, int nq, int sk);
-int sparse_attn(const va_attn_args& a, cudaStream_t stream);
+int sparse_attn(const va_attn_args& a, cudaStream_t stream, bool own_blocks = false, int first_tile = 0, int seq_len = 0);
 int qk_norm_rope(const va_norm_rope_args& a, cudaStream_t stream);
 int qk_head_norm_rope(const va_head_norm_rope_args& a, cudaStream_t stream);
 
@@ -47,9 +47,9 @@ static inline bool bk_ok(int bk) { return bk == 16 || bk == 32 || bk == 64 || bk
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 struct PrefillPlan {
-  int nq_total, nqc_max, blk_width, step;  // step: query rows handled per launch
+  int nq_total, nqc_max, step;  // step: query rows handled per launch
   int64_t capacity;
-  size_t off_avg, off_cnt, off_idx, off_bcnt, off_bidx, off_mask, mask_bytes, total;
+  size_t off_avg, off_cnt, off_idx, off_mask, mask_bytes, total;
 };
 
 static inline size_t budget_of(const va_prefill_args& a) {
@@ -69,7 +69,6 @@ static int plan_prefill(const va_prefill_args& a, PrefillPlan& pl, size_t single
   const size_t bh = (size_t)a.batch * a.heads;
   const int chunk = a.chunk_size < a.sq ? a.chunk_size : a.sq;
   pl.nq_total = (a.sq + a.pq - 1) / a.pq;
-  pl.blk_width = a.causal ? 2 * (a.pq / 64) : 1;
   pl.capacity = (a.sk + 3) / 4 * 4;
   // one launch per stage for the whole sequence when its index lists fit the budget
   const bool single = bh * (size_t)pl.nq_total * (size_t)pl.capacity * 4 <= single_pass_budget;
@@ -78,8 +77,6 @@ static int plan_prefill(const va_prefill_args& a, PrefillPlan& pl, size_t single
   size_t off = 0;
   pl.off_avg = off;  off = align_up(off + bh * pl.nqc_max * kHeadDim * 2, 256);
   pl.off_cnt = off;  off = align_up(off + bh * pl.nqc_max * 4, 256);
-  pl.off_bcnt = off; off = align_up(off + bh * pl.nqc_max * 4, 256);
-  pl.off_bidx = off; off = align_up(off + bh * pl.nqc_max * pl.blk_width * 4, 256);
   pl.mask_bytes = select_workspace_bytes(a.batch, a.heads, a.kv_heads, pl.nqc_max, a.sk);
   pl.off_mask = off; off = align_up(off + pl.mask_bytes, 256);
   pl.off_idx = off;  off = align_up(off + bh * pl.nqc_max * (size_t)pl.capacity * 4, 256);
@@ -235,8 +232,6 @@ static int run_prefill(const va_prefill_args* a, size_t single_pass_budget, va_s
   void* avg = ws + pl.off_avg;
   int32_t* cnt = reinterpret_cast<int32_t*>(ws + pl.off_cnt);
   int32_t* idx = reinterpret_cast<int32_t*>(ws + pl.off_idx);
-  int32_t* bcnt = reinterpret_cast<int32_t*>(ws + pl.off_bcnt);
-  int32_t* bidx = reinterpret_cast<int32_t*>(ws + pl.off_bidx);
   const int bh = a->batch * a->heads;
   const size_t esz = 2;
 
@@ -263,10 +258,6 @@ static int run_prefill(const va_prefill_args* a, size_t single_pass_budget, va_s
     sa.workspace = ws + pl.off_mask; sa.workspace_bytes = pl.mask_bytes;
     if (int rc = select(sa, stream)) return rc;
 
-    block_tables_kernel<<<(bh * nqc + 255) / 256, 256, 0, stream>>>(bh, a->sq, a->pq, a->causal, i / a->pq, nqc, bcnt,
-                                                                    bidx);
-    if (cudaGetLastError() != cudaSuccess) return VA_ERR_CUDA;
-
     va_attn_args aa{};
     aa.dtype = a->dtype; aa.batch = a->batch; aa.heads = a->heads; aa.kv_heads = a->kv_heads;
     aa.sq = sqc; aa.head_dim = a->head_dim; aa.pq = a->pq;
@@ -274,11 +265,10 @@ static int run_prefill(const va_prefill_args* a, size_t single_pass_budget, va_s
     aa.sk = a->causal ? (int)(kend < a->sk ? kend : a->sk) : a->sk;  // VecAttention.py:107-108
     aa.causal = a->causal; aa.q_offset = i;
     aa.q = qc; aa.k = a->k; aa.v = a->v; aa.out = oc;
-    aa.blk_count = bcnt; aa.blk_idx = bidx; aa.blk_stride = pl.blk_width;
     aa.col_count = cnt; aa.col_idx = idx; aa.col_stride = pl.capacity;
     aa.softmax_scale = 0.f;
     aa.status = a->status;
-    if (int rc = sparse_attn(aa, stream)) return rc;
+    if (int rc = sparse_attn(aa, stream, true, i / a->pq, a->sq)) return rc;
 
     if (a->col_count_out) {
       if (cudaMemcpy2DAsync(a->col_count_out + i / a->pq, (size_t)pl.nq_total * 4, cnt, (size_t)nqc * 4,

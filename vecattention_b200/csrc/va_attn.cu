@@ -9,7 +9,8 @@ int launch_attn64(const AttnParams& p, int dtype, int batch, cudaStream_t stream
 int launch_attn128(const AttnParams& p, int dtype, int batch, cudaStream_t stream);  // va_attn128.cu
 bool launch_dense128(const AttnParams& p, int dtype, int batch, cudaStream_t stream, int* rc);
 
-int sparse_attn(const va_attn_args& a, cudaStream_t stream) {
+// own_blocks: the tables' place is taken by the operator's own rule (see AttnParams)
+int sparse_attn(const va_attn_args& a, cudaStream_t stream, bool own_blocks, int first_tile, int seq_len) {
   AttnParams p;
   p.q = a.q.ptr; p.k = a.k.ptr; p.v = a.v.ptr; p.out = a.out.ptr;
   p.q_sb = a.q.stride_b; p.q_sh = a.q.stride_h; p.q_ss = a.q.stride_s;
@@ -21,6 +22,7 @@ int sparse_attn(const va_attn_args& a, cudaStream_t stream) {
   p.v_row_bytes = row_bytes(p.v_ss);
   p.blk_count = a.blk_idx ? a.blk_count : nullptr;
   p.blk_idx = a.blk_idx; p.blk_stride = a.blk_stride;
+  p.own_blocks = own_blocks; p.first_tile = first_tile; p.seq_len = seq_len;
   p.col_count = a.col_count; p.col_idx = a.col_idx; p.col_stride = a.col_stride;
   p.status = a.status;
   p.lse = a.lse;

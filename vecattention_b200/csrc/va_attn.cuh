@@ -27,6 +27,9 @@ struct AttnParams {
   // from tiles that need no tables, rows [vis_begin, vis_end) the sparse attention of their tile; `nq` then counts
   // the table tiles (rows [0, vis_end)) and the grid has the dense tiles behind them.
   int vis_on, vis_begin, vis_end;
+  // The operator's own dense blocks, which follow from the tile's number and need no table: under the causal rule the first
+  // tile's and the tile's own, else none.  Tile t of this launch is tile first_tile + t of a sequence of seq_len rows.
+  int own_blocks, first_tile, seq_len;
   int group;  // heads whose tiles are listed together: tile 0 of each of them, then tile 1 of each, ...
 };
 
@@ -38,6 +41,21 @@ __device__ __forceinline__ void place(const AttnParams& p, int tiles, uint32_t x
   head = (int)(first + in_group % n);
   x = in_group / n;
   tile = p.causal ? tiles - 1 - (int)x : (int)x;
+}
+
+// The operator's dense 64-key blocks of query tile t (of PQ rows): how many, and where block j starts.
+template <int PQ>
+__device__ __forceinline__ int own_block_count(const AttnParams& p, int t) {
+  constexpr int n = PQ / 64;
+  if (!p.causal) return 0;
+  t += p.first_tile;
+  if (t == 0) return (min(p.seq_len, PQ) + 63) / 64;
+  return n + min(n, (p.seq_len - t * PQ + 63) / 64);
+}
+template <int PQ>
+__device__ __forceinline__ int own_block_start(const AttnParams& p, int t, int j) {
+  constexpr int n = PQ / 64;
+  return j < n ? j * 64 : (p.first_tile + t) * PQ + (j - n) * 64;
 }
 
 }  // namespace va

@@ -212,14 +212,16 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn64_kernel(const AttnPa
           // requested before the counts are known; a tile with dense blocks, which come first in slot order, fetches again
 #pragma unroll
           for (int i = 0; i < 8; ++i) raw[i] = !dense && i * 32 + lane < p.col_stride ? ldg_nc(col + i * 32 + lane) : 0;
-          const int nblk = dense ? (row_end - 1) / 64 + 1 : (p.blk_count ? __ldg(p.blk_count + trow) : 0);
+          const int nblk = dense ? (row_end - 1) / 64 + 1
+                                 : (p.own_blocks ? own_block_count<PQ>(p, tile) : (p.blk_count ? __ldg(p.blk_count + trow) : 0));
           const int ncol = dense ? 0 : __ldg(p.col_count + trow);
           if (nblk > 0) {
             const int32_t* blk = dense ? nullptr : p.blk_idx + trow * p.blk_stride;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int slot = i * 32 + lane, ci = slot - nblk * 64;
-              if (slot < nblk * 64) raw[i] = dense ? (slot >> 6) << 6 : ldg_nc(blk + (slot >> 6));
+              if (slot < nblk * 64)
+                raw[i] = dense ? (slot >> 6) << 6 : (p.own_blocks ? own_block_start<PQ>(p, tile, slot >> 6) : ldg_nc(blk + (slot >> 6)));
               else raw[i] = ci < ncol ? ldg_nc(col + ci) : 0;
             }
           }
