@@ -188,3 +188,35 @@ def test_selection_in_segments(heads, kv, s, pq, bk, group, causal, chunk_tiles)
         for t in range(0, q.shape[2], step):
             part = lists(q[:, h:h + 1, t:t + step], k[:, kh:kh + 1], t, gap[h:h + 1])
             assert torch.equal(part, whole[:, h:h + 1, t:t + step])
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("pq,bk", [(64, 16), (128, 128)])
+def test_calls_in_a_row_and_in_a_graph(pq, bk, causal):
+    """The kernels of a call are launched before the ones ahead of them have ended.  Calls on alternating inputs that share one
+    workspace and one output, without waiting in between, and a captured call that is replayed on new inputs, give what
+    each gives alone."""
+    from vecattention_b200 import VecAttention_prefill
+    g = torch.Generator(device=DEV).manual_seed(pq)
+    sets = [[torch.randn(1, n, 1500, 128, generator=g, device=DEV).bfloat16() for n in (6, 2, 2)] for _ in range(3)]
+    run = lambda x, **kw: VecAttention_prefill(*x, 0.8, pq, bk, 1, causal, 16384, **kw)  # noqa: E731
+    alone = []
+    for x in sets:
+        alone.append(run(x).clone())
+        torch.cuda.synchronize()
+    out, kept = torch.empty_like(sets[0][0]), []
+    for i in range(30):
+        run(sets[i % 3], out=out)
+        kept.append(out.clone())
+    for i, o in enumerate(kept):
+        assert torch.equal(o, alone[i % 3])
+    x = [t.clone() for t in sets[0]]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(x, out=out)
+        run(x, out=out)
+    for i in (1, 2, 0):
+        for a, b in zip(x, sets[i]):
+            a.copy_(b)
+        graph.replay()
+        assert torch.equal(out, alone[i])

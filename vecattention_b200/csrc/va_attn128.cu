@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
   __shared__ float m_row_s[2][128];           // [chunk parity][row]: the rows' shared reference maxima (exp2 domain)
   __shared__ float fin_s[256];                // [group * 128 + row]: row sums, added in the epilogue
 
+  wait_for_previous();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int tile, h;
   place(p, (int)gridDim.x, blockIdx.x, blockIdx.y, tile, h);
@@ -511,8 +512,7 @@ int launch(const AttnParams& p, const DenseMaps& maps, int tiles, int batch, cud
   // per-device attribute; setting it on every launch keeps multi-device processes correct
   auto kern = attn128_kernel<DT, DENSE>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess) return VA_ERR_CUDA;
-  kern<<<dim3(tiles, p.heads, batch), kThreads, kSmem, stream>>>(p, maps);
-  return cudaGetLastError() == cudaSuccess ? VA_OK : VA_ERR_CUDA;
+  return launch_after(kern, dim3(tiles, p.heads, batch), kThreads, kSmem, stream, p, maps) == cudaSuccess ? VA_OK : VA_ERR_CUDA;
 }
 
 }  // namespace

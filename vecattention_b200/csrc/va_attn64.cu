@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn64_kernel(const AttnPa
     tmem_alloc(&tmem_base_s, 256);
     tmem_relinquish();
   }
+  wait_for_previous();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -626,8 +627,7 @@ int launch(const AttnParams& p, int batch, cudaStream_t stream) {
   int tiles = p.nq;
   if (p.vis_on) tiles += (p.vis_begin + 63) / 64 + (p.sq - p.vis_end + 63) / 64;  // the dense tiles before and after
   dim3 grid(tiles, p.heads, batch);
-  kern<<<grid, kThreads, kSmem, stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? VA_OK : VA_ERR_CUDA;
+  return launch_after(kern, grid, kThreads, kSmem, stream, p) == cudaSuccess ? VA_OK : VA_ERR_CUDA;
 }
 
 }  // namespace

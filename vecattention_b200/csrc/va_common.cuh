@@ -106,4 +106,30 @@ __device__ __forceinline__ int ldg_nc(const int32_t* p) {
 // pull the 128-byte line at `p` into L2 (no register result, no wait)
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// ---- launches that overlap their predecessor's end -----------------------------------------------
+// A kernel launched with launch_after may be scheduled while the kernel before it in the stream is still running, once
+// every CTA of that one has let it (let_next_start) or ended.  It must not touch memory, not even read an argument's target, and
+// no CTA of it may end before wait_for_previous, which returns when the kernel before has ended and its writes are visible:
+// so the order of all effects is that of plain launches, also for the kernels after it.  What overlaps is the launch itself
+// and the setting up before the wait (barriers, tensor memory).
+// A call that is waited for: 4 heads x 2048 tokens 62.0 -> 57.2 us, 28/4 heads x 9001 360 -> 354, 20 011 around a vision span 817 -> 810;
+// in a row of calls 34.2 -> 33.5 for the first, which the host limits.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 }  // namespace va

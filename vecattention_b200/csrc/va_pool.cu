@@ -20,6 +20,7 @@ __global__ void __launch_bounds__(128) pool_q_kernel(const typename Elem<DT>::T*
   const int valid = min(PQ, seq_len - row0);
   const typename Elem<DT>::T* base = q + b * sb + h * sh + (int64_t)row0 * ss + c * 8;
 
+  let_next_start();
   uint4 raw[R];
 #pragma unroll
   for (int i = 0; i < R; ++i) {

@@ -338,6 +338,8 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
   __shared__ WalkShared wsh;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  wait_for_previous();
+  let_next_start();
   const int nrows = p.rep * p.nq;
   // ---- this CTA's row block and segment ----
   const int blocks = p.rows_pad / kRows;
@@ -523,6 +525,8 @@ __device__ __forceinline__ int warp_prefix_sum(int x) {
 template <int BK>
 __global__ void __launch_bounds__(kExpandWarps * 32) select_expand_kernel(const SelectParams p, int64_t total_rows) {
   __shared__ __align__(16) int32_t stage_s[kExpandWarps][1024 + kFlushFrom];
+  wait_for_previous();
+  let_next_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t row = (int64_t)blockIdx.x * kExpandWarps + warp;  // = (b * heads + h) * nq + tile
   if (row >= total_rows) return;
@@ -605,12 +609,12 @@ int launch_bk(const SelectParams& p, const CUtensorMap& kmap, int batch, cudaStr
   // per-device attribute; setting it on every launch keeps multi-device processes correct
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess) return VA_ERR_CUDA;
   if (p.plan.ctas > 0) {
-    kern<<<p.plan.ctas, kThreads, kSmem, stream>>>(kmap, p);
-    if (cudaGetLastError() != cudaSuccess) return VA_ERR_CUDA;
+    if (launch_after(kern, dim3(p.plan.ctas), kThreads, kSmem, stream, kmap, p) != cudaSuccess) return VA_ERR_CUDA;
   }
   const int64_t total_rows = (int64_t)batch * p.heads * p.nq;
-  select_expand_kernel<BK><<<(unsigned)((total_rows + kExpandWarps - 1) / kExpandWarps), kExpandWarps * 32, 0, stream>>>(p, total_rows);
-  return cudaGetLastError() == cudaSuccess ? VA_OK : VA_ERR_CUDA;
+  const cudaError_t e = launch_after(select_expand_kernel<BK>, dim3((unsigned)((total_rows + kExpandWarps - 1) / kExpandWarps)),
+                                     kExpandWarps * 32, 0, stream, p, total_rows);
+  return e == cudaSuccess ? VA_OK : VA_ERR_CUDA;
 }
 
 template <int DT>
