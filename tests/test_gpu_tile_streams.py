@@ -220,3 +220,27 @@ def test_calls_in_a_row_and_in_a_graph(pq, bk, causal):
             a.copy_(b)
         graph.replay()
         assert torch.equal(out, alone[i])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads,kv,s", [(300, 100, 200), (40, 40, 1400), (30, 5, 1281)])
+def test_dense_tiles_that_follow_one_another(dtype, heads, kv, s):
+    """Several dense tiles for every SM, of 1 to 11 chunks, with scores that grow along the keys, so that the running maximum
+    moves and partial results are rescaled.  A value that is not finite in the last row reaches only the last block."""
+    from vecattention_b200.dispatch import Full_prefill
+    g = torch.Generator(device=DEV).manual_seed(s)
+    q = torch.randn(1, heads, s, 128, generator=g, device=DEV)
+    k = torch.randn(1, kv, s, 128, generator=g, device=DEV)
+    q[..., 0] = 8.0
+    k[..., 0] = torch.linspace(0, 40.0, s, device=DEV)
+    q, k = q.to(dtype), k.to(dtype)
+    v = torch.randn(1, kv, s, 128, generator=g, device=DEV).to(dtype)
+    out = Full_prefill(q, k, v)
+    rep = heads // kv
+    ref = torch.nn.functional.scaled_dot_product_attention(q.float(), k.float().repeat_interleave(rep, 1),
+                                                           v.float().repeat_interleave(rep, 1), is_causal=True)
+    _close(out, ref)
+    v[:, :, -1] = math.inf
+    again = Full_prefill(q, k, v)
+    whole = (s - 1) // 64 * 64
+    assert torch.equal(again[:, :, :whole], out[:, :, :whole]) and not again[:, :, -1].isfinite().any()

@@ -1,5 +1,5 @@
 // Vector-sparse flash attention: launch parameters from the C ABI's argument struct, and the choice of the
-// kernel by query-tile height (q_pooling_size 64: va_attn64.cu, 128: va_attn128.cu).
+// kernel by query-tile height (q_pooling_size 64: va_attn64.cu, 128: va_attn128.cu; dense rows: va_dense128.cu).
 #include "va_common.cuh"
 #include "va_attn.cuh"
 
@@ -7,7 +7,7 @@ namespace va {
 
 int launch_attn64(const AttnParams& p, int dtype, int batch, cudaStream_t stream);   // va_attn64.cu
 int launch_attn128(const AttnParams& p, int dtype, int batch, cudaStream_t stream);  // va_attn128.cu
-bool launch_dense128(const AttnParams& p, int dtype, int batch, cudaStream_t stream, int* rc);
+bool launch_dense128(const AttnParams& p, int dtype, int batch, cudaStream_t stream, int* rc);  // va_dense128.cu
 
 // own_blocks: the tables' place is taken by the operator's own rule (see AttnParams)
 int sparse_attn(const va_attn_args& a, cudaStream_t stream, bool own_blocks, int first_tile, int seq_len) {
@@ -42,7 +42,7 @@ int sparse_attn(const va_attn_args& a, cudaStream_t stream, bool own_blocks, int
   const int64_t fit = kv_bytes < (64 << 20) ? (64 << 20) / kv_bytes : 1;
   const int groups = (int)((a.kv_heads + fit - 1) / fit);
   p.group = (a.kv_heads + groups - 1) / groups * p.rep;
-  if (p.vis_on && p.vis_begin >= p.vis_end) {  // every row is dense: 128-row tiles on streamed K and V take 0.50 ms where
+  if (p.vis_on && p.vis_begin >= p.vis_end) {  // every row is dense: 128-row tiles on streamed K and V take 0.47 ms where
     // gathered 64-row tiles took 0.86 (28 query heads on 4 KV heads, 8192 tokens).  A composition with sparse rows keeps its
     // dense tiles in the 64-row launch: they are few, and a launch of their own would leave most SMs idle.
     int rc;

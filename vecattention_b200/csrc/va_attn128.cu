@@ -1,7 +1,7 @@
-// Flash attention with 128-row query tiles on tcgen05 MMAs with M = 128: vector-sparse (q_pooling_size 128) and dense.
+// Vector-sparse flash attention for q_pooling_size 128 on tcgen05 MMAs with M = 128.
 //
 // One CTA per query tile of 128 rows; keys are taken 128 at a time, from the tile's dense 64-key blocks and then its
-// selected-column list (row gather), or, in the dense form, from key 0 up to the tile's last row.  S = Q K^T and
+// selected-column list (row gather).  S = Q K^T and
 // O += P V are tcgen05.mma with M = 128, N = 128: accumulator row r lives in TMEM lane r.  P is the PV product's A operand
 // in tensor memory, so it never passes through shared memory: of the traffic of a chunk (K and V written 64 KB, Q and K
 // read by S 64 KB, V read by PV 32 KB) the 64 KB that P's store and operand read were are gone.
@@ -12,9 +12,8 @@
 //              it by more than 2^8; the value is shared by both groups through shared memory), writes
 //              P = exp2(S*scale - m) in the input dtype into its group's P buffer in tensor memory and rescales the row
 //              of O in the rare chunks where the maximum moved.
-//   warps 8-15  sparse: K (8-11) and V (12-15) gather producers, cp.async 16-byte pieces of the selected rows into rings
-//              of 128-byte-swizzled operand tiles (3 K stages, 2 V stages).  Dense: the tiles are contiguous, one
-//              thread each streams K and V by TMA into the same rings.  Warps 8-11 copy the Q tile in both.
+//   warps 8-15  K (8-11) and V (12-15) gather producers, cp.async 16-byte pieces of the selected rows into rings
+//              of 128-byte-swizzled operand tiles (3 K stages, 2 V stages).  Warps 8-11 copy the Q tile too.
 //   warps 16,17  MMA issuers (one thread each): warp 16 issues S_j = Q K_j^T into one of two S
 //              buffers, warp 17 issues O += P_j V_j; the tensor pipe works on S_{j+1} while the
 //              softmax of chunk j runs.
@@ -22,15 +21,14 @@
 // Every wait is a bounded mbarrier wait; a timeout sets VA_STATUS_TIMEOUT and unwinds the CTA.
 //
 // What bounds it: the softmax groups, three quarters of whose time is work (64 + 128 special-function and fp32 issue slots
-// and the tensor-memory latencies between them; both groups of a scheduler share its special-function unit), then, in the
-// sparse form, the gather beside them.  Measured on one B200 with the former kernel (P in shared memory, eight warps in
-// lockstep on one chunk, 64-row gathered tiles for dense rows): 32 heads x 32 K tokens causal at the reference's default
-// arguments 1.97 -> 1.69 ms for the whole operator (1.75 while the gather multiplied 64-bit row offsets); dense causal, 28 query heads on 4 KV heads, 8192 tokens, 0.855 -> 0.504 ms
-// (560 -> 950 TFLOP/s; 0.519 while the dense form too read a quarter of the scores twice for want of registers).
+// and the tensor-memory latencies between them; both groups of a scheduler share its special-function unit), then
+// the gather beside them.  Measured on one B200 with the former kernel (P in shared memory, eight warps in
+// lockstep on one chunk): 32 heads x 32 K tokens causal at the reference's default
+// arguments 1.97 -> 1.69 ms for the whole operator (1.75 while the gather multiplied 64-bit row offsets).
+// Tiles that run on in a CTA, as with 64 rows, with two K stages and the one O buffer that tensor memory has room for: 1.53 -> 1.64 ms.
 #include "va_common.cuh"
 #include "va_sm100.cuh"
 #include "va_attn.cuh"
-#include "va_tmap.cuh"
 
 namespace va {
 
@@ -45,12 +43,10 @@ constexpr int kVStages = 2;
 constexpr int kThreads = 576;
 // Registers per thread: the kernel is launched with 96 (the most 18 warps can all have); the two producer warpgroups
 // hand 40 each back and the two softmax warpgroups take them: 256 * 56 + 256 * 136 + 64 * 96 = 576 * 96.
-// The dense kernel's producers only start TMA copies: they hand 72 each back, and a softmax thread can hold a whole row.
 constexpr int kLaunchRegs = 96;
-constexpr int kProducerRegs = 56, kSoftmaxRegs = 136, kDenseProducerRegs = 24, kDenseSoftmaxRegs = 168;
+constexpr int kProducerRegs = 56, kSoftmaxRegs = 136;
 // the softmax warps can only take what the producer warps hand back: the sum must fit the launch allocation
 static_assert(256 * kProducerRegs + 256 * kSoftmaxRegs + 64 * kLaunchRegs <= kThreads * kLaunchRegs, "setmaxnreg pool");
-static_assert(256 * kDenseProducerRegs + 256 * kDenseSoftmaxRegs + 64 * kLaunchRegs <= kThreads * kLaunchRegs, "setmaxnreg pool");
 constexpr size_t kSmem = 1024 + (size_t)kTileBytes * (1 + kKStages + kVStages);  // Q, K ring, V ring
 constexpr float kRescaleThreshold = 8.0f;                                        // log2 units
 
@@ -64,15 +60,8 @@ __device__ __forceinline__ void reg_alloc() { asm volatile("setmaxnreg.inc.sync.
 template <int N>
 __device__ __forceinline__ void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
-// Tensor maps of K and V for the dense kernel (rows of 128 elements, boxes of 128 rows by 64 elements).
-struct DenseMaps {
-  CUtensorMap k, v;
-};
-
-// DENSE: full causal attention of all rows (one sequence for queries and keys): a tile's keys are 0, 1, 2, ... up to its
-// last row, so K and V tiles are contiguous and two threads stream them by TMA.
-template <int DT, bool DENSE>
-__global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p, const __grid_constant__ DenseMaps maps) {
+template <int DT>
+__global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p) {
   using T = typename Elem<DT>::T;
   constexpr int PQ = 128;
   extern __shared__ unsigned char smem_raw[];
@@ -90,10 +79,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
   place(p, (int)gridDim.x, blockIdx.x, blockIdx.y, tile, h);
   const int b = blockIdx.z;
   const int hkv = h / p.rep;
-  const int row0 = tile * PQ, row_end = DENSE ? min(p.sq, row0 + PQ) : p.sq;  // rows at or past row_end do not exist
-  const int64_t trow = DENSE ? 0 : ((int64_t)b * p.heads + h) * p.nq + tile;
-  const int nblk = DENSE ? 0 : (p.own_blocks ? own_block_count<PQ>(p, tile) : (p.blk_count ? __ldg(p.blk_count + trow) : 0));
-  const int ncol = DENSE ? row_end : __ldg(p.col_count + trow);
+  const int row0 = tile * PQ, row_end = p.sq;  // rows at or past row_end do not exist
+  const int64_t trow = ((int64_t)b * p.heads + h) * p.nq + tile;
+  const int nblk = p.own_blocks ? own_block_count<PQ>(p, tile) : (p.blk_count ? __ldg(p.blk_count + trow) : 0);
+  const int ncol = __ldg(p.col_count + trow);
   const int nslots = nblk * 64 + ncol;
   const int nchunks = (nslots + kChunk - 1) / kChunk;
   T* ob = static_cast<T*>(p.out) + b * p.o_sb + h * p.o_sh;
@@ -115,11 +104,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
   if (tid == 0) {
     mbar_init(&bars.qfull, 128);  // per producer thread: one arrival, made by the hardware when the thread's copies have landed
     for (int s = 0; s < kKStages; ++s) {
-      mbar_init(&bars.kfull[s], DENSE ? 1 : 128);
+      mbar_init(&bars.kfull[s], 128);
       mbar_init(&bars.kempty[s], 1);
     }
     for (int s = 0; s < kVStages; ++s) {
-      mbar_init(&bars.vfull[s], DENSE ? 1 : 128);
+      mbar_init(&bars.vfull[s], 128);
       mbar_init(&bars.vempty[s], 1);
     }
     for (int s = 0; s < 2; ++s) {
@@ -148,13 +137,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
 
   if (warp >= 8 && warp < 16) {
     // ======================= gather producers (warps 8-11: K and the Q tile, warps 12-15: V) =======================
-    reg_dealloc<DENSE ? kDenseProducerRegs : kProducerRegs>();
+    reg_dealloc<kProducerRegs>();
     const bool is_v = warp >= 12;
     const int pt = is_v ? tid - 384 : tid - 256;
     const T* qb = static_cast<const T*>(p.q) + b * p.q_sb + h * p.q_sh;
     const T* kb = static_cast<const T*>(p.k) + b * p.k_sb + hkv * p.k_sh;
     const T* vb = static_cast<const T*>(p.v) + b * p.v_sb + hkv * p.v_sh;
-    const int32_t* blk = DENSE ? nullptr : p.blk_idx + trow * p.blk_stride;
+    const int32_t* blk = p.blk_idx + trow * p.blk_stride;
     const int32_t* col = p.col_idx + trow * p.col_stride;
     if (!is_v) {
 #pragma unroll
@@ -165,96 +154,75 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
       }
       cp_async_arrive_noinc(&bars.qfull);
     }
-    if constexpr (DENSE) {
-      if ((warp & 3) == 0 && lane == 0) {
-        unsigned char* ring = is_v ? v_s : k_s;
-        uint64_t *full = is_v ? bars.vfull : bars.kfull, *empty = is_v ? bars.vempty : bars.kempty;
-        const int stages = is_v ? kVStages : kKStages;
-        const CUtensorMap* map = is_v ? &maps.v : &maps.k;
-        int stage = 0, j = 0;
-        uint32_t round = 0;
-        for (; j < nchunks; ++j) {
-          if (!mbar_wait(&empty[stage], round ^ 1)) { timed_out = true; break; }
-          mbar_expect_tx(&full[stage], kTileBytes);
-          const uint32_t dst = smem_addr(ring) + (uint32_t)stage * kTileBytes;
-          tma_load_4d(dst, map, 0, j * kChunk, hkv, b, &full[stage]);
-          tma_load_4d(dst + kTileBytes / 2, map, 64, j * kChunk, hkv, b, &full[stage]);
-          if (++stage == stages) { stage = 0; round ^= 1; }
-        }
-        if (timed_out)  // copies still in flight must land before the CTA's memory is given back
-          for (int i = max(0, j - stages); i < j; ++i) mbar_wait(&full[i % stages], (i / stages) & 1);
+    // Copy geometry.  A warp covers two key rows per instruction: lanes 0-15 the sixteen 16-byte
+    // pieces of row rbase + 8 i, lanes 16-31 those of the next row.  Because the rows of one thread
+    // differ by multiples of 8, its swizzled piece position is the same in all of them and the
+    // shared-memory destinations are one base address plus i * 1024.
+    // Each lane fetches ONE key index per chunk (that of row rbase + 8 * (lane & 15)), two chunks
+    // ahead; the sixteen indices a thread needs are then exchanged through shared memory.
+    const int pw = (pt >> 5), hi = lane >> 4, c = lane & 15;
+    const int rbase = 2 * pw + hi;
+    const uint32_t dst_off = tile_off(128, rbase, c);
+    const int my_slot = rbase + 8 * c;
+    auto fetch_raw = [&](int j) -> int {
+      const int slot = j * kChunk + my_slot;
+      const int ci = min(max(slot - nblk * 64, 0), max(ncol - 1, 0));
+      if (p.own_blocks && slot < nblk * 64) return own_block_start<PQ>(p, tile, slot >> 6);
+      return ldg_nc(slot < nblk * 64 ? blk + (slot >> 6) : col + ci);
+    };
+    auto decode = [&](int j, int raw) -> int {
+      const int slot = j * kChunk + my_slot;
+      const int key = slot < nblk * 64 ? raw + (slot & 63) : (slot < nslots ? raw : -1);
+      return (key >= 0 && key < p.sk) ? key : -1;
+    };
+    // through a small exchange array of the warp: one store and four 16-byte loads per thread instead of sixteen
+    // shuffles; two buffers, so the next chunk's stores cannot overtake this chunk's loads
+    int* xk = xk_s[warp - 8][0];
+    auto spread = [&](int j, int key, int (&out)[16]) {
+      int* buf = xk + (j & 1) * 32;
+      buf[lane] = max(key, 0);  // an unused slot copies row 0: its scores are masked and its P is zero
+      __syncwarp();
+      const int4* src = reinterpret_cast<const int4*>(buf + (lane & 16));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int4 q4 = src[i];
+        out[4 * i] = q4.x; out[4 * i + 1] = q4.y; out[4 * i + 2] = q4.z; out[4 * i + 3] = q4.w;
       }
-    } else {
-      // Copy geometry.  A warp covers two key rows per instruction: lanes 0-15 the sixteen 16-byte
-      // pieces of row rbase + 8 i, lanes 16-31 those of the next row.  Because the rows of one thread
-      // differ by multiples of 8, its swizzled piece position is the same in all of them and the
-      // shared-memory destinations are one base address plus i * 1024.
-      // Each lane fetches ONE key index per chunk (that of row rbase + 8 * (lane & 15)), two chunks
-      // ahead; the sixteen indices a thread needs are then exchanged through shared memory.
-      const int pw = (pt >> 5), hi = lane >> 4, c = lane & 15;
-      const int rbase = 2 * pw + hi;
-      const uint32_t dst_off = tile_off(128, rbase, c);
-      const int my_slot = rbase + 8 * c;
-      auto fetch_raw = [&](int j) -> int {
-        const int slot = j * kChunk + my_slot;
-        const int ci = min(max(slot - nblk * 64, 0), max(ncol - 1, 0));
-        if (p.own_blocks && slot < nblk * 64) return own_block_start<PQ>(p, tile, slot >> 6);
-        return ldg_nc(slot < nblk * 64 ? blk + (slot >> 6) : col + ci);
-      };
-      auto decode = [&](int j, int raw) -> int {
-        const int slot = j * kChunk + my_slot;
-        const int key = slot < nblk * 64 ? raw + (slot & 63) : (slot < nslots ? raw : -1);
-        return (key >= 0 && key < p.sk) ? key : -1;
-      };
-      // through a small exchange array of the warp: one store and four 16-byte loads per thread instead of sixteen
-      // shuffles; two buffers, so the next chunk's stores cannot overtake this chunk's loads
-      int* xk = xk_s[warp - 8][0];
-      auto spread = [&](int j, int key, int (&out)[16]) {
-        int* buf = xk + (j & 1) * 32;
-        buf[lane] = max(key, 0);  // an unused slot copies row 0: its scores are masked and its P is zero
-        __syncwarp();
-        const int4* src = reinterpret_cast<const int4*>(buf + (lane & 16));
+    };
+    auto copy_tile = [&](unsigned char* tile_s, const T* base, int64_t stride, int row_bytes, const int (&keys)[16], uint64_t* full) {
+      const uint32_t dst = smem_addr(tile_s) + dst_off;
+      const char* src = reinterpret_cast<const char*>(base + c * 8);
+      if (row_bytes != 0) {  // one 32-bit multiplication into the 64-bit address per row
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int4 q4 = src[i];
-          out[4 * i] = q4.x; out[4 * i + 1] = q4.y; out[4 * i + 2] = q4.z; out[4 * i + 3] = q4.w;
-        }
-      };
-      auto copy_tile = [&](unsigned char* tile_s, const T* base, int64_t stride, int row_bytes, const int (&keys)[16], uint64_t* full) {
-        const uint32_t dst = smem_addr(tile_s) + dst_off;
-        const char* src = reinterpret_cast<const char*>(base + c * 8);
-        if (row_bytes != 0) {  // one 32-bit multiplication into the 64-bit address per row
+        for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * row_bytes);
+      } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * row_bytes);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * (stride * 2));
-        }
-        cp_async_arrive_noinc(full);
-      };
-      int keys[16];
-      int raw0 = fetch_raw(0), raw1 = nchunks > 1 ? fetch_raw(1) : 0;
-      for (int j = 0; j < nchunks && !timed_out; ++j) {
-        const int key = decode(j, raw0);
-        raw0 = raw1;
-        if (j + 2 < nchunks) raw1 = fetch_raw(j + 2);
-        if (!is_v) {
-          keys_s[j & 7][my_slot] = key;
-          // unused slots, and keys that some row of the tile may not see, make the chunk take the masking pass
-          const bool flag = key < 0 || (p.causal && key > p.q_offset + row0);
-          const int any = __any_sync(0xffffffffu, flag);
-          if (lane == 0) mask_s[j & 7][pw] = any;
-        }
-        spread(j, key, keys);
-        if (!is_v) {
-          const int ks = j % kKStages, ku = j / kKStages;
-          if (!mbar_wait(&bars.kempty[ks], (ku & 1) ^ 1)) { timed_out = true; break; }
-          copy_tile(k_s + (size_t)ks * kTileBytes, kb, p.k_ss, p.k_row_bytes, keys, &bars.kfull[ks]);
-        } else {
-          const int vs = j % kVStages, vu = j / kVStages;
-          if (!mbar_wait(&bars.vempty[vs], (vu & 1) ^ 1)) { timed_out = true; break; }
-          copy_tile(v_s + (size_t)vs * kTileBytes, vb, p.v_ss, p.v_row_bytes, keys, &bars.vfull[vs]);
-        }
+        for (int i = 0; i < 16; ++i) cp_async16_full(dst + i * 1024, src + (int64_t)keys[i] * (stride * 2));
+      }
+      cp_async_arrive_noinc(full);
+    };
+    int keys[16];
+    int raw0 = fetch_raw(0), raw1 = nchunks > 1 ? fetch_raw(1) : 0;
+    for (int j = 0; j < nchunks && !timed_out; ++j) {
+      const int key = decode(j, raw0);
+      raw0 = raw1;
+      if (j + 2 < nchunks) raw1 = fetch_raw(j + 2);
+      if (!is_v) {
+        keys_s[j & 7][my_slot] = key;
+        // unused slots, and keys that some row of the tile may not see, make the chunk take the masking pass
+        const bool flag = key < 0 || (p.causal && key > p.q_offset + row0);
+        const int any = __any_sync(0xffffffffu, flag);
+        if (lane == 0) mask_s[j & 7][pw] = any;
+      }
+      spread(j, key, keys);
+      if (!is_v) {
+        const int ks = j % kKStages, ku = j / kKStages;
+        if (!mbar_wait(&bars.kempty[ks], (ku & 1) ^ 1)) { timed_out = true; break; }
+        copy_tile(k_s + (size_t)ks * kTileBytes, kb, p.k_ss, p.k_row_bytes, keys, &bars.kfull[ks]);
+      } else {
+        const int vs = j % kVStages, vu = j / kVStages;
+        if (!mbar_wait(&bars.vempty[vs], (vu & 1) ^ 1)) { timed_out = true; break; }
+        copy_tile(v_s + (size_t)vs * kTileBytes, vb, p.v_ss, p.v_row_bytes, keys, &bars.vfull[vs]);
       }
     }
     cp_async_commit();
@@ -289,18 +257,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
           tc_fence_after();
           // a K16 step is 2048 bytes further down the V tile (descriptor addresses count 16 bytes)
           const uint64_t vd = vd0 + (uint64_t)(s * (kTileBytes >> 4));
-          // Dense: the first 64 rows of the tile see none of the last 64 keys, and their weights for them, exact zeros, would
-          // still turn an Inf or NaN in V into a NaN.  That half of the product goes to an accumulator of its own, where the S
-          // of this chunk was (read by all of its group before P was complete, and no S follows); the epilogue adds it to the
-          // other 64 rows.  0.442 ms before and after (28 query heads
-          // on 4 KV heads, 8192 tokens).
-          const bool last = DENSE && j == nchunks - 1;
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const bool apart = last && ks >= 4;
-            umma_ts(apart ? t_s0 + (uint32_t)(pb * 128) : t_o, t_p0 + (uint32_t)(pb * 64 + ks * 8), vd + ks * 128, idesc_pv,
-                    (apart ? ks > 4 : j > 0 || ks > 0) ? 1u : 0u);
-          }
+          for (int ks = 0; ks < 8; ++ks)
+            umma_ts(t_o, t_p0 + (uint32_t)(pb * 64 + ks * 8), vd + ks * 128, idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
           umma_commit(&bars.vempty[s]);
           umma_commit(&bars.pempty[pb]);
           if (j == nchunks - 1) umma_commit(&bars.ofull);
@@ -315,7 +274,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
     // a thread of either group owns a whole row.  The reference maximum of a row is one value shared by both groups
     // (m_row_s): the decision for chunk j starts from the value left by chunk j - 1, so all P tiles and O stay on one
     // scale.
-    reg_alloc<DENSE ? kDenseSoftmaxRegs : kSoftmaxRegs>();
+    reg_alloc<kSoftmaxRegs>();
     const int grp = warp >> 2, qtr = warp & 3;
     const uint32_t lane_base = (uint32_t)(qtr * 32) << 16;
     const int row = qtr * 32 + lane;
@@ -327,13 +286,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
       const int* keys = keys_s[j & 7];
       if (!mbar_wait(&bars.sfull[grp], ub & 1)) { timed_out = true; break; }
       tc_fence_after();
-      bool masked;
-      if constexpr (DENSE) {
-        masked = (j + 1) * kChunk - 1 > row0;
-      } else {
-        const int4 mk = *reinterpret_cast<const int4*>(mask_s[j & 7]);
-        masked = (mk.x | mk.y | mk.z | mk.w) != 0;
-      }
+      const int4 mk = *reinterpret_cast<const int4*>(mask_s[j & 7]);
+      const bool masked = (mk.x | mk.y | mk.z | mk.w) != 0;
       // ---- the row's maximum.  Beside the gather producers a whole row of 128 scores does not fit the registers: the
       // first 32 are then read again below, the other 96 stay (v[1..3]) ----
       const uint32_t t_s = t_s0 + (uint32_t)(grp * 128) + lane_base;
@@ -343,8 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
         if (!masked) return;  // kept out of the arithmetic loops: a branch per element would serialise them
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
-          const int first = j * kChunk + c * 32 + i;
-          const int4 k4 = DENSE ? make_int4(first, first + 1, first + 2, first + 3) : *reinterpret_cast<const int4*>(keys + c * 32 + i);
+          const int4 k4 = *reinterpret_cast<const int4*>(keys + c * 32 + i);
           if ((uint32_t)k4.x > last_key) v[c][i] = 0xff800000u;  // -inf; an unused slot's key is -1
           if ((uint32_t)k4.y > last_key) v[c][i + 1] = 0xff800000u;
           if ((uint32_t)k4.z > last_key) v[c][i + 2] = 0xff800000u;
@@ -358,26 +311,14 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
       };
       tmem_ld32(t_s, v[0]);
       tmem_ld32(t_s + 32, v[1]);
-      if constexpr (DENSE) {
-        tmem_ld32(t_s + 64, v[2]);
-        tmem_ld32(t_s + 96, v[3]);
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(&bars.sempty[grp]);  // the S buffer has been read
-        hide(0);
-        top(0);
-        hide(1);
-        top(1);
-      } else {
-        tmem_wait_ld();
-        hide(0);
-        top(0);
-        tmem_ld32(t_s + 64, v[2]);
-        tmem_ld32(t_s + 96, v[3]);
-        hide(1);
-        top(1);
-        tmem_wait_ld();
-      }
+      tmem_wait_ld();
+      hide(0);
+      top(0);
+      tmem_ld32(t_s + 64, v[2]);
+      tmem_ld32(t_s + 96, v[3]);
+      hide(1);
+      top(1);
+      tmem_wait_ld();
       hide(2);
       hide(3);
       top(2);
@@ -434,14 +375,12 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
         }
       };
       expo(1);
-      if constexpr (!DENSE) tmem_ld32(t_s, v[0]);
+      tmem_ld32(t_s, v[0]);
       expo(2);
-      if constexpr (!DENSE) {
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(&bars.sempty[grp]);  // the S buffer has been read
-        hide(0);
-      }
+      tmem_wait_ld();
+      tc_fence_before();
+      mbar_arrive(&bars.sempty[grp]);  // the S buffer has been read
+      hide(0);
       expo(3);
       expo(0);
       const float2 la = halves(ls[0]), lb = halves(ls[1]);
@@ -472,18 +411,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
         tmem_ld32(t_o + lane_base + grp * 64, o[0]);
         tmem_ld32(t_o + lane_base + grp * 64 + 32, o[1]);
         tmem_wait_ld();
-        if constexpr (DENSE) {
-          if (qtr >= 2) {  // rows 64 and up: the last 64 keys' part
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              uint32_t x[32];
-              tmem_ld32(t_s0 + (uint32_t)((jl & 1) * 128) + lane_base + grp * 64 + c * 32, x);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) o[c][i] = __float_as_uint(__uint_as_float(o[c][i]) + __uint_as_float(x[i]));
-            }
-          }
-        }
         if (row_ok) {
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -507,33 +434,18 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
   if (warp == 16) tmem_dealloc(tmem, 512);
 }
 
-template <int DT, bool DENSE>
-int launch(const AttnParams& p, const DenseMaps& maps, int tiles, int batch, cudaStream_t stream) {
+template <int DT>
+int launch(const AttnParams& p, int batch, cudaStream_t stream) {
   // per-device attribute; setting it on every launch keeps multi-device processes correct
-  auto kern = attn128_kernel<DT, DENSE>;
+  auto kern = attn128_kernel<DT>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess) return VA_ERR_CUDA;
-  return launch_after(kern, dim3(tiles, p.heads, batch), kThreads, kSmem, stream, p, maps) == cudaSuccess ? VA_OK : VA_ERR_CUDA;
+  return launch_after(kern, dim3(p.nq, p.heads, batch), kThreads, kSmem, stream, p) == cudaSuccess ? VA_OK : VA_ERR_CUDA;
 }
 
 }  // namespace
 
 int launch_attn128(const AttnParams& p, int dtype, int batch, cudaStream_t stream) {
-  const DenseMaps none{};
-  return dtype == VA_BF16 ? launch<VA_BF16, false>(p, none, p.nq, batch, stream) : launch<VA_FP16, false>(p, none, p.nq, batch, stream);
-}
-
-// false: the tensors cannot be described by a tensor map (nothing has been launched)
-bool launch_dense128(const AttnParams& p, int dtype, int batch, cudaStream_t stream, int* rc) {
-  DenseMaps maps;
-  const int kv_heads = p.heads / p.rep, bf16 = dtype == VA_BF16;
-  auto forward = [&](int64_t sb, int64_t sh, int64_t ss) { return ss > 0 && (kv_heads == 1 || sh > 0) && (batch == 1 || sb > 0); };
-  if (!forward(p.k_sb, p.k_sh, p.k_ss) || !forward(p.v_sb, p.v_sh, p.v_ss)) return false;  // repeated or reversed rows
-  if (!encode_rows_map(&maps.k, bf16, p.k, batch, kv_heads, p.sk, p.k_sb, p.k_sh, p.k_ss, kChunk) ||
-      !encode_rows_map(&maps.v, bf16, p.v, batch, kv_heads, p.sk, p.v_sb, p.v_sh, p.v_ss, kChunk))
-    return false;
-  const int tiles = (p.sq + 127) / 128;
-  *rc = bf16 ? launch<VA_BF16, true>(p, maps, tiles, batch, stream) : launch<VA_FP16, true>(p, maps, tiles, batch, stream);
-  return true;
+  return dtype == VA_BF16 ? launch<VA_BF16>(p, batch, stream) : launch<VA_FP16>(p, batch, stream);
 }
 
 }  // namespace va

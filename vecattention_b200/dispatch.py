@@ -38,9 +38,9 @@ def Full_prefill(query_states: torch.Tensor, key_states: torch.Tensor, value_sta
     if causal and q_off < 0:
         raise VecAttentionArgumentError("causal dense attention needs at least as many keys as queries")
     if causal and q_off == 0:  # vision-slice mode without a sparse row: no table is read
-        none = torch.zeros(b, h, nq, dtype=torch.int32, device=dev)
-        return _sparse_attn_bhsd(query_states, key_states, value_states, 64, None, None, none,
-                                 torch.zeros(b, h, nq, 4, dtype=torch.int32, device=dev), True, vision=(sq, sq))
+        return _sparse_attn_bhsd(query_states, key_states, value_states, 64, None, None,
+                                 torch.empty(b, h, nq, dtype=torch.int32, device=dev),
+                                 torch.empty(b, h, nq, 4, dtype=torch.int32, device=dev), True, vision=(sq, sq))
     last_key = (torch.clamp(q_off + (torch.arange(nq, device=dev) + 1) * 64, max=q_off + sq) - 1) if causal else \
         torch.full((nq,), sk - 1, device=dev)
     count = (last_key // 64 + 1).to(torch.int32)
