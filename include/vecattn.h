@@ -64,6 +64,10 @@ typedef struct {
 } va_pool_args;
 int va_pool_q(const va_pool_args* args, va_stream_t stream);
 
+/* ---- thresholds on the device ---------------------------------------------------------------
+ * gaps[i] = -log(threshold[i] + 1e-9) in fp32, i < n (spattn/src/VecAttention.py:48-52), in one launch. */
+int va_threshold_gaps(const float* threshold, int32_t n, float* gaps, va_stream_t stream);
+
 /* ---- important-vector (key column) selection -------------------------------------------------
  * Replaces fuse_qk_softmax_minp_wo_causal(avg_q_chunk, k, avg_q_chunk_offset, gap, causal,
  * q_pooling_size, k_local_size, wo_initial, group_k_block),
@@ -296,7 +300,8 @@ typedef struct {
 int va_qk_head_norm_rope(const va_head_norm_rope_args* args, va_stream_t stream);
 
 const char* va_status_string(int code);
-/* 100 * major + minor of this interface (201: va_attn_args gained the vision_* fields, va_qk_head_norm_rope added). */
+/* 100 * major + minor of this interface (201: va_attn_args gained the vision_* fields, va_qk_head_norm_rope added;
+ * 202: va_threshold_gaps added). */
 int va_version(void);
 
 #ifdef __cplusplus

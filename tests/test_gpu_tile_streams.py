@@ -244,3 +244,19 @@ def test_dense_tiles_that_follow_one_another(dtype, heads, kv, s):
     again = Full_prefill(q, k, v)
     whole = (s - 1) // 64 * 64
     assert torch.equal(again[:, :, :whole], out[:, :, :whole]) and not again[:, :, -1].isfinite().any()
+
+
+@pytest.mark.parametrize("n", [1, 28, 127, 128, 129, 70000])
+def test_gaps_of_thresholds(n):
+    """Gaps from thresholds on the device: the bits of the expression they stand for, also at 0, 1, infinity, NaN and below
+    zero, and of a part of a larger tensor.  Other types and layouts take that expression itself."""
+    from vecattention_b200.api import _gap_of
+    dev = torch.device(DEV, torch.cuda.current_device())
+    g = torch.Generator(device=DEV).manual_seed(n)
+    t = torch.rand(n + 5, generator=g, device=DEV) ** 3
+    t[5:][:5] = torch.tensor([0.0, 1.0, math.inf, math.nan, -1.0], device=DEV)[:min(n, 5)]
+    for x in (t[5:], t[5:].double(), t[5:].half(), t.expand(3, n + 5)[:, 5:], t[5:].cpu()):
+        want = -torch.log(x.to(dev) + 1e-9)
+        got = _gap_of(x, dev)
+        assert got.dtype == want.dtype and got.shape == want.shape
+        assert torch.equal(got.nan_to_num(7.0, 8.0, 9.0), want.nan_to_num(7.0, 8.0, 9.0)) and torch.equal(got.isnan(), want.isnan())

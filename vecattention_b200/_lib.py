@@ -15,7 +15,7 @@ VA_STATUS_OVERFLOW = 1
 VA_STATUS_TIMEOUT = 2
 
 # every symbol include/vecattn.h declares
-EXPORTS = ("va_pool_q", "va_select", "va_select_workspace_bytes", "va_sparse_attn", "va_sparse_attn_workspace_bytes",
+EXPORTS = ("va_pool_q", "va_threshold_gaps", "va_select", "va_select_workspace_bytes", "va_sparse_attn", "va_sparse_attn_workspace_bytes",
            "va_block_tables", "va_prefill_workspace_bytes", "va_prefill", "va_prefill_static", "va_prefill_static_fits",
            "va_selftest_wait_timeout", "va_qk_norm_rope", "va_qk_head_norm_rope", "va_status_string", "va_version")
 VA_SINGLE_PASS_INDEX_BYTES_DEFAULT = 4 << 30
@@ -99,6 +99,7 @@ def lib() -> C.CDLL:
         if not hasattr(handle, name):
             raise RuntimeError(f"{LIB_PATH} does not export {name}")
     handle.va_pool_q.argtypes = [C.POINTER(PoolArgs), C.c_void_p]
+    handle.va_threshold_gaps.argtypes = [C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p]
     handle.va_select.argtypes = [C.POINTER(SelectArgs), C.c_void_p]
     handle.va_sparse_attn.argtypes = [C.POINTER(AttnArgs), C.c_void_p]
     handle.va_select_workspace_bytes.argtypes = [C.POINTER(SelectArgs), C.POINTER(C.c_size_t)]

@@ -94,6 +94,19 @@ def _check(code: int) -> None:
         raise RuntimeError(f"libvecattn: {msg} (status {code})")
 
 
+def _gap_of(threshold: Union[float, torch.Tensor], dev: torch.device) -> Union[float, torch.Tensor]:
+    """-log(threshold + 1e-9): a float, or a tensor on ``dev``."""
+    if not isinstance(threshold, torch.Tensor):
+        return -math.log(threshold + 1e-9, math.e)
+    t = threshold.to(dev)
+    if t.dtype != torch.float32 or not t.is_contiguous() or t.requires_grad or not 0 < t.numel() < 1 << 31:
+        return -torch.log(t + 1e-9)
+    gap = torch.empty_like(t)
+    with _on(dev):
+        _check(L.lib().va_threshold_gaps(t.data_ptr(), t.numel(), gap.data_ptr(), _stream()))
+    return gap
+
+
 def _gap_args(gap: Union[float, torch.Tensor], batch: int, heads: int, device) -> Tuple[float, Optional[torch.Tensor], int]:
     """float gap -> (gap, None, 0); tensor gap -> (0, fp32 device tensor, batch stride)."""
     if isinstance(gap, torch.Tensor):
@@ -310,10 +323,7 @@ def VecAttention_prefill(
         raise VecAttentionArgumentError("causal selection needs q_pooling_size % k_local_size == 0")
 
     # gap = -log(threshold)  (spattn/src/VecAttention.py:48-52)
-    if isinstance(threshold, torch.Tensor):
-        gap = -torch.log(threshold.to(dev) + 1e-9)
-    else:
-        gap = -math.log(threshold + 1e-9, math.e)
+    gap = _gap_of(threshold, dev)
     gapf, gaps, gstride = _gap_args(gap, b, h, dev)
 
     q, k, v = _rows_ok(query_states), _rows_ok(key_states), _rows_ok(value_states)

@@ -36,6 +36,13 @@ __global__ void block_tables_kernel(int bh, int seq_len, int pq, int causal, int
   }
 }
 
+// The selection's gaps from thresholds: the three elementwise launches that this takes with a tensor library were 7 of the 320 us
+// of a 9001-token prompt with a threshold per head.
+__global__ void threshold_gaps_kernel(const float* __restrict__ threshold, int n, float* __restrict__ gaps) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) gaps[i] = -logf(__fadd_rn(threshold[i], 1e-9f));
+}
+
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 static inline bool strides_ok(int64_t sb, int64_t sh, int64_t ss) { return sb % 8 == 0 && sh % 8 == 0 && ss % 8 == 0; }
 template <class TT> static inline int check_tensor(const TT& t) {
@@ -89,7 +96,7 @@ using namespace va;
 
 extern "C" {
 
-int va_version(void) { return 201; }  // 201: va_attn_args gained the vision fields; va_qk_head_norm_rope
+int va_version(void) { return 202; }  // 201: va_attn_args gained the vision fields; va_qk_head_norm_rope.  202: va_threshold_gaps
 
 const char* va_status_string(int code) {
   switch (code) {
@@ -104,6 +111,14 @@ const char* va_status_string(int code) {
     case VA_ERR_PARAM: return "parameters rejected (q_pooling_size must be 64 or 128, chunk_size a multiple of it, causal needs q_pooling_size % k_local_size == 0 and Sq == Sk)";
     default: return "unknown status";
   }
+}
+
+int va_threshold_gaps(const float* threshold, int32_t n, float* gaps, va_stream_t stream) {
+  if (!threshold || !gaps) return VA_ERR_NULL;
+  if (n <= 0) return VA_ERR_SHAPE;
+  if (((reinterpret_cast<uintptr_t>(threshold) | reinterpret_cast<uintptr_t>(gaps)) & 3u) != 0) return VA_ERR_ALIGN;
+  threshold_gaps_kernel<<<(n - 1) / 128 + 1, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(threshold, n, gaps);
+  return cudaGetLastError() == cudaSuccess ? VA_OK : VA_ERR_CUDA;
 }
 
 int va_pool_q(const va_pool_args* a, va_stream_t stream) {

@@ -17,7 +17,7 @@ from typing import Optional, Tuple, Union
 
 import torch
 
-from .api import (VecAttention_prefill, VecAttentionArgumentError, _sparse_attn_bhsd, average_vector, block_tables,
+from .api import (VecAttention_prefill, VecAttentionArgumentError, _gap_of, _sparse_attn_bhsd, average_vector, block_tables,
                   fuse_qk_softmax_minp_wo_causal)
 
 _DENSE_TILE = 64  # query rows per tile of the dense passes
@@ -96,8 +96,7 @@ def VecAttention_prefill_vision(
         # shows in the rows the causal rule treats specially), then one attention launch over all rows
         if threshold is None:
             raise VecAttentionArgumentError("threshold is required")
-        gap = -torch.log(threshold.to(query_states.device) + 1e-9) if isinstance(threshold, torch.Tensor) \
-            else -math.log(threshold + 1e-9, math.e)
+        gap = _gap_of(threshold, query_states.device)
         if chunk_size % q_pooling_size != 0:
             raise VecAttentionArgumentError("chunk_size must be a multiple of q_pooling_size")
         avg = average_vector(query_states[:, :, :end], 64)
