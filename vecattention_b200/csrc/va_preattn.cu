@@ -29,7 +29,7 @@ __device__ __forceinline__ typename Elem<DT>::T from_double(double x) {
 // ---- the rotation of a pair, rounded once ----
 // x = a c - b s rounded once to the 16-bit type is what the double-precision expression gives.  Its conversions and the
 // rounding from double cost the kernel, which is bound by issue slots, more than the norm did, so nearly all pairs are
-// done in fp32 with the same result (40 heads, 75 600 tokens: 0.995 -> 0.82 ms, 3.15 -> 3.8 TB/s; a branch per pair instead of
+// done in fp32 with the same result (40 heads, 75 600 tokens: 0.995 -> 0.82 ms; a branch per pair instead of
 // one per piece of four: 0.886):
 //  * Kahan's product sum (w = b s; f = a c - w; t = f + (w - b s), both fma exact to their last rounding) is within
 //    1.5 units in the last place of x (Jeannerod, Louvet, Muller, "Further analysis of Kahan's algorithm for the accurate
@@ -105,22 +105,25 @@ __device__ __forceinline__ void turn(const float (&y)[8], const float (&c)[4], c
 // shared memory (one block barrier).  Few registers, hence some thirty warps resident per SM: enough outstanding
 // memory, which one CTA per row with one piece or two per thread in flight was not (2.4 TB/s).  A CTA holds as many
 // whole rows as fit eight warps.
+// Bound by issue slots (71 %), and a row has only sixteen pairs per lane: what is done once a row counts.  With a 64-bit remainder, two
+// divisions by W and a loop over the row's partial sums it took 0.813 ms at 40 heads x 75 600 tokens in bf16 (0.843 in fp16), without
+// them 0.714 (0.725), 4.3 TB/s; 12 heads x 30 000 0.114 -> 0.103.
 constexpr int NP = 4;  // pieces per lane
 // ROTATE: the call has tables.  The norm alone is a kernel of its own: with the rotation's registers and branches around it,
 // it took 0.612 ms (0.579 before the rotation was done in fp32), alone 0.521 (40 heads, 75 600 tokens).
 template <int DT, bool ROTATE>
-__global__ void __launch_bounds__(256, 4) qk_norm_rope_rows_kernel(const va_norm_rope_args a, int64_t rows, int W, int rows_per_cta) {
+__global__ void __launch_bounds__(256, 4) qk_norm_rope_rows_kernel(const va_norm_rope_args a, uint32_t rows) {
   using T = typename Elem<DT>::T;
-  __shared__ float part[8];  // [row of the CTA * W + warp of the row]
+  __shared__ __align__(16) float part[8][8];  // [row of the CTA][warp of the row], zeros behind the last
   const bool is_k = blockIdx.y == 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int rsub = warp / W, wsub = warp % W;
-  const int64_t token = (int64_t)blockIdx.x * rows_per_cta + rsub;  // b * seq_len + s
-  const bool live = token < rows;
-  const int s = (int)((live ? token : 0) % a.seq_len);
+  // a block is 32 W x rows threads: no division by W, and 32-bit arithmetic up to the addresses
+  const int lane = threadIdx.x & 31, W = blockDim.x >> 5, wsub = threadIdx.x >> 5, rsub = threadIdx.y;
+  const uint32_t at = blockIdx.x * blockDim.y + rsub;  // b * seq_len + s
+  const bool live = at < rows;
+  const uint32_t token = live ? at : 0;
   const int hidden = (is_k ? a.kv_heads : a.heads) * kHeadDim;
-  const T* x = static_cast<const T*>(is_k ? a.k : a.q) + (live ? token : 0) * (is_k ? a.k_row_stride : a.q_row_stride);
-  T* y = static_cast<T*>(is_k ? a.k_out : a.q_out) + (live ? token : 0) * (is_k ? a.k_out_row_stride : a.q_out_row_stride);
+  const T* x = static_cast<const T*>(is_k ? a.k : a.q) + (int64_t)token * (is_k ? a.k_row_stride : a.q_row_stride);
+  T* y = static_cast<T*>(is_k ? a.k_out : a.q_out) + (int64_t)token * (is_k ? a.k_out_row_stride : a.q_out_row_stride);
   const T* w = static_cast<const T*>(is_k ? a.k_weight : a.q_weight);
   const int pieces = live ? hidden / 8 : 0;
 
@@ -144,15 +147,16 @@ __global__ void __launch_bounds__(256, 4) qk_norm_rope_rows_kernel(const va_norm
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   if (W > 1) {
-    if (lane == 0) part[rsub * W + wsub] = ss;
+    if (lane == 0) part[rsub][wsub] = ss;
+    if (wsub == 0 && lane >= W && lane < 8) part[rsub][lane] = 0.f;
     __syncthreads();
-    ss = 0.f;
-    for (int i = 0; i < W; ++i) ss += part[rsub * W + i];  // the same order in every warp of the row
+    const float4 a0 = *reinterpret_cast<const float4*>(part[rsub]), a1 = *reinterpret_cast<const float4*>(part[rsub] + 4);
+    ss = ((((((a0.x + a0.y) + a0.z) + a0.w) + a1.x) + a1.y) + a1.z) + a1.w;  // the same order in every warp of the row
   }
   const float rstd = w ? 1.0f / sqrtf(ss / (float)hidden + a.eps) : 1.0f;  // no weight: no normalisation
   const uint64_t rstd2 = pair2(rstd, rstd);
 
-  const int rs = s - a.rope_skip;  // row of the cos / sin tables; the first rope_skip tokens are not rotated
+  const int rs = (int)(a.batch == 1 ? token : token % (uint32_t)a.seq_len) - a.rope_skip;  // row of the cos / sin tables; the first rope_skip tokens are not rotated
   const bool rotate = ROTATE && live && rs >= 0;
   float cc[4] = {}, sv[4] = {};
   if (rotate) {  // a lane's pieces lie 32 W pieces apart, whole heads: all of them sit at the same place of their head
@@ -207,7 +211,7 @@ int launch_rows_dt(const va_norm_rope_args& a, cudaStream_t stream) {
   const int per = 8 / W;
   dim3 grid((unsigned)((rows + per - 1) / per), 2, 1);
   auto kern = a.cos ? qk_norm_rope_rows_kernel<DT, true> : qk_norm_rope_rows_kernel<DT, false>;
-  kern<<<grid, 32 * W * per, 0, stream>>>(a, rows, W, per);
+  kern<<<grid, dim3(32 * W, per), 0, stream>>>(a, (uint32_t)rows);
   return cudaGetLastError() == cudaSuccess ? VA_OK : VA_ERR_CUDA;
 }
 
