@@ -481,7 +481,7 @@ def _launches_per_step(wl):
     idx_all_bytes = wl.batch * wl.heads * wl.nq * ((wl.seq_len + 3) // 4 * 4) * 4
     free, _ = torch.cuda.mem_get_info()
     n_chunks = 1 if idx_all_bytes <= min(32 << 30, int(free * 0.4)) else math.ceil(wl.seq_len / wl.chunk_size)
-    return n_chunks * 5  # pool + selection (two kernels) + block tables + attention per pass
+    return n_chunks * 4  # pool + selection (two kernels) + attention per pass
 
 
 def _parity_on_cpu_sample(va, cwl, q_rows, thr, ref_out, ref_counts, dev):
