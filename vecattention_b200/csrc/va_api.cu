@@ -11,15 +11,15 @@ int sparse_attn(const va_attn_args& a, cudaStream_t stream, bool own_blocks = fa
 int qk_norm_rope(const va_norm_rope_args& a, cudaStream_t stream);
 int qk_head_norm_rope(const va_head_norm_rope_args& a, cudaStream_t stream);
 
-// dense-block tables of query tiles [tile_off, tile_off + nqc) written as a contiguous (BH, nqc) slice
-__global__ void block_tables_kernel(int bh, int seq_len, int pq, int causal, int tile_off, int nqc,
-                                    int32_t* __restrict__ blk_count, int32_t* __restrict__ blk_idx) {
+// dense-block tables of all query tiles, for callers of the stages (va_prefill's attention derives them: own_block_count)
+__global__ void block_tables_kernel(int bh, int seq_len, int pq, int causal, int32_t* __restrict__ blk_count,
+                                    int32_t* __restrict__ blk_idx) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= bh * nqc) return;
+  const int nq = (seq_len + pq - 1) / pq;
+  if (i >= bh * nq) return;
   const int n = pq / 64;
   const int width = causal ? 2 * n : 1;
-  const int t = tile_off + i % nqc;
-  const int nq = (seq_len + pq - 1) / pq;
+  const int t = i % nq;
   int32_t* row = blk_idx + (int64_t)i * width;
   if (!causal) {
     blk_count[i] = 0;
@@ -220,7 +220,7 @@ int va_block_tables(int32_t batch, int32_t heads, int32_t seq_len, int32_t pq, i
   const int64_t n = (int64_t)batch * heads * nq;
   if (n > 0x7fffffff) return VA_ERR_SHAPE;
   block_tables_kernel<<<(unsigned)((n + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      batch * heads, seq_len, pq, causal, 0, nq, blk_count, blk_idx);
+      batch * heads, seq_len, pq, causal, blk_count, blk_idx);
   return cudaGetLastError() == cudaSuccess ? VA_OK : VA_ERR_CUDA;
 }
 
@@ -300,7 +300,7 @@ int va_prefill(const va_prefill_args* a, va_stream_t stream) {
 }
 
 // ---- the operator for callers that cannot allocate device memory -----------------------------
-// The scratch of the prefill (pooled queries, per-tile counts, block tables and the selected-
+// The scratch of the prefill (pooled queries, per-tile counts, keep bits and the selected-
 // column index lists) lives in this fixed array instead of a caller-supplied workspace.  It is
 // part of the loaded module, so every GPU that loads the library holds it until the process exits.
 static __device__ __align__(256) unsigned char g_static_scratch[VA_STATIC_SCRATCH_BYTES];
