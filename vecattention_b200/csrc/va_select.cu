@@ -645,10 +645,13 @@ size_t select_workspace_bytes(int batch, int heads, int kv_heads, int nq, int sk
 }
 
 // Cut the work into CTAs so that the SMs finish together: the number of segments per row block is the one with the least
-// estimated time, in tiles.  A tile that only feeds the running maximum costs kFeed of one with keep bits, a CTA kSetUp tiles
-// (it loads its rows, fills and drains its pipeline: 3 us).
+// estimated time, in tiles.  A tile that only feeds the running maximum costs kFeed of one with keep bits (more than its
+// instructions' share: with many segments the CTAs stream K from L2 at the same time), a CTA kSetUp tiles
+// (it loads its rows, fills and drains its pipeline: 3 us).  Whole calls of one group with 0.55 / 0.62 / 0.70: 3 heads x 55 000 tokens 1185 /
+// 1159 / 1112 us, 4 x 55 000 1439 / 1425 / 1414, 5 x 75 600 2629 / 2622 / 2624, 3 x 118 800 3222 / 3203 / 3242 (1167, 1445, 2680 and 3309 with up to four equal
+// segments).
 static void make_plan(SelectParams& p, int batch, int bk) {
-  constexpr double kFeed = 0.55, kSetUp = 5.0;
+  constexpr double kFeed = 0.70, kSetUp = 5.0;
   Plan& pl = p.plan;
   int sms = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
