@@ -286,8 +286,8 @@ static int run_prefill(const va_prefill_args* a, size_t single_pass_budget, va_s
     if (int rc = sparse_attn(aa, stream, true, i / a->pq, a->sq)) return rc;
 
     if (a->col_count_out) {
-      if (cudaMemcpy2DAsync(a->col_count_out + i / a->pq, (size_t)pl.nq_total * 4, cnt, (size_t)nqc * 4,
-                            (size_t)nqc * 4, bh, cudaMemcpyDeviceToDevice, stream) != cudaSuccess)
+      if (!succeeded(cudaMemcpy2DAsync(a->col_count_out + i / a->pq, (size_t)pl.nq_total * 4, cnt, (size_t)nqc * 4,
+                                       (size_t)nqc * 4, bh, cudaMemcpyDeviceToDevice, stream)))
         return VA_ERR_CUDA;
     }
   }
@@ -336,7 +336,7 @@ int va_prefill_static(const va_prefill_args* a, va_stream_t stream) {
   // call (a host-side lookup once the module is loaded on the device), so nothing stale survives a
   // cudaDeviceReset or a re-created context.
   void* ptr = nullptr;
-  if (cudaGetSymbolAddress(&ptr, g_static_scratch) != cudaSuccess || !ptr) return VA_ERR_CUDA;
+  if (!succeeded(cudaGetSymbolAddress(&ptr, g_static_scratch)) || !ptr) return VA_ERR_CUDA;
   va_prefill_args b = *a;
   b.workspace = ptr;
   b.workspace_bytes = VA_STATIC_SCRATCH_BYTES;

@@ -438,8 +438,8 @@ template <int DT>
 int launch(const AttnParams& p, int batch, cudaStream_t stream) {
   // per-device attribute; setting it on every launch keeps multi-device processes correct
   auto kern = attn128_kernel<DT>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess) return VA_ERR_CUDA;
-  return launch_after(kern, dim3(p.nq, p.heads, batch), kThreads, kSmem, stream, p) == cudaSuccess ? VA_OK : VA_ERR_CUDA;
+  if (!succeeded(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem))) return VA_ERR_CUDA;
+  return launch_after(kern, dim3(p.nq, p.heads, batch), kThreads, kSmem, stream, p) ? VA_OK : VA_ERR_CUDA;
 }
 
 }  // namespace

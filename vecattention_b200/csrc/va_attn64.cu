@@ -623,11 +623,11 @@ template <int DT>
 int launch(const AttnParams& p, int batch, cudaStream_t stream) {
   // per-device attribute; setting it on every launch keeps multi-device processes correct
   auto kern = p.vis_on ? sparse_attn64_kernel<DT, true> : sparse_attn64_kernel<DT, false>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess) return VA_ERR_CUDA;
+  if (!succeeded(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem))) return VA_ERR_CUDA;
   int tiles = p.nq;
   if (p.vis_on) tiles += (p.vis_begin + 63) / 64 + (p.sq - p.vis_end + 63) / 64;  // the dense tiles before and after
   dim3 grid(tiles, p.heads, batch);
-  return launch_after(kern, grid, kThreads, kSmem, stream, p) == cudaSuccess ? VA_OK : VA_ERR_CUDA;
+  return launch_after(kern, grid, kThreads, kSmem, stream, p) ? VA_OK : VA_ERR_CUDA;
 }
 
 }  // namespace

@@ -106,6 +106,14 @@ __device__ __forceinline__ int ldg_nc(const int32_t* p) {
 // pull the 128-byte line at `p` into L2 (no register result, no wait)
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// ---- errors of the runtime ------------------------------------------------------------------------
+// A failed call's error stays with the thread until cudaGetLastError takes it, and the plain launches are checked with
+// cudaGetLastError: a call that answers for itself takes its error back, or the next launch would be reported as failed.
+inline bool succeeded(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return e == cudaSuccess;
+}
+
 // ---- launches that overlap their predecessor's end -----------------------------------------------
 // A kernel launched with launch_after may be scheduled while the kernel before it in the stream is still running, once
 // every CTA of that one has let it (let_next_start) or ended.  It must not touch memory, not even read an argument's target, and
@@ -118,7 +126,7 @@ __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontr
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... Params, typename... Args>
-inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, Args... args) {
+inline bool launch_after(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -129,7 +137,7 @@ inline cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, unsigned t
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  return succeeded(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
 }
 
 }  // namespace va

@@ -458,8 +458,8 @@ template <int DT>
 int launch(const AttnParams& p, const DenseMaps& maps, int tiles, int batch, cudaStream_t stream) {
   // per-device attribute; setting it on every launch keeps multi-device processes correct
   auto kern = dense128_kernel<DT>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess) return VA_ERR_CUDA;
-  return launch_after(kern, dim3(tiles, p.heads, batch), kThreads, kSmem, stream, p, maps) == cudaSuccess ? VA_OK : VA_ERR_CUDA;
+  if (!succeeded(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem))) return VA_ERR_CUDA;
+  return launch_after(kern, dim3(tiles, p.heads, batch), kThreads, kSmem, stream, p, maps) ? VA_OK : VA_ERR_CUDA;
 }
 
 }  // namespace

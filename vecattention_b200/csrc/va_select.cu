@@ -607,14 +607,13 @@ int launch_bk(const SelectParams& p, const CUtensorMap& kmap, int batch, cudaStr
   if (kTile % group == 0) kern = select_mask_kernel<DT, BK, kInTiles>;
   else if (group % kTile == 0) kern = select_mask_kernel<DT, BK, kAtTiles>;
   // per-device attribute; setting it on every launch keeps multi-device processes correct
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem) != cudaSuccess) return VA_ERR_CUDA;
+  if (!succeeded(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem))) return VA_ERR_CUDA;
   if (p.plan.ctas > 0) {
-    if (launch_after(kern, dim3(p.plan.ctas), kThreads, kSmem, stream, kmap, p) != cudaSuccess) return VA_ERR_CUDA;
+    if (!launch_after(kern, dim3(p.plan.ctas), kThreads, kSmem, stream, kmap, p)) return VA_ERR_CUDA;
   }
   const int64_t total_rows = (int64_t)batch * p.heads * p.nq;
-  const cudaError_t e = launch_after(select_expand_kernel<BK>, dim3((unsigned)((total_rows + kExpandWarps - 1) / kExpandWarps)),
-                                     kExpandWarps * 32, 0, stream, p, total_rows);
-  return e == cudaSuccess ? VA_OK : VA_ERR_CUDA;
+  const dim3 grid((unsigned)((total_rows + kExpandWarps - 1) / kExpandWarps));
+  return launch_after(select_expand_kernel<BK>, grid, kExpandWarps * 32, 0, stream, p, total_rows) ? VA_OK : VA_ERR_CUDA;
 }
 
 template <int DT>
@@ -654,7 +653,7 @@ static void make_plan(SelectParams& p, int batch, int bk) {
   constexpr double kFeed = 0.70, kSetUp = 5.0;
   Plan& pl = p.plan;
   int sms = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (!succeeded(cudaGetDevice(&dev)) || !succeeded(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev))) sms = 148;
   const int blocks = p.rows_pad / kRows, t0 = (p.wo_initial ? p.pq : 0) / kTile;
   const int all = (p.sk + kTile - 1) / kTile;
   pl.heads = p.kv_heads * batch;

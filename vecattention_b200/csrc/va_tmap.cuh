@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "va_common.cuh"
+
 namespace va {
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -16,7 +18,7 @@ inline EncodeTiledFn tmap_encoder() {
   static EncodeTiledFn fn = [] {
     void* f = nullptr;
     cudaDriverEntryPointQueryResult qr;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &qr) != cudaSuccess ||
+    if (!succeeded(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &qr)) ||
         qr != cudaDriverEntryPointSuccess)
       f = nullptr;
     return reinterpret_cast<EncodeTiledFn>(f);
