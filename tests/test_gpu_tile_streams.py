@@ -222,6 +222,50 @@ def test_calls_in_a_row_and_in_a_graph(pq, bk, causal):
         assert torch.equal(out, alone[i])
 
 
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("pq,bk", [(64, 16), (128, 128)])
+def test_selection_and_attention_in_a_row_on_the_same_buffers(pq, bk, causal):
+    """Selection and attention through the C interface, again and again on alternating inputs with one set of scratch, counts and
+    lists, with nothing launched between them and nothing waited for: every kernel overlaps the end of the one that
+    writes what it reads.  Each call gives what it gives alone."""
+    import ctypes as C
+    from vecattention_b200 import _lib as L
+    from vecattention_b200.api import _check, _stream, _t4, average_vector, block_tables
+    heads, kv, s = 6, 2, 1500
+    nq, cap = -(-s // pq), (s + 3) // 4 * 4
+    g = torch.Generator(device=DEV).manual_seed(pq)
+    sets = [[torch.randn(1, n, s, 128, generator=g, device=DEV).bfloat16() for n in (heads, kv, kv)] for _ in range(3)]
+    avg = [average_vector(x[0], pq) for x in sets]
+    bcnt, bidx = block_tables(1, heads, s, pq, causal, DEV)
+    count = torch.empty(1, heads, nq, dtype=torch.int32, device=DEV)
+    index = torch.empty(1, heads, nq, cap, dtype=torch.int32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    outs = [torch.empty_like(sets[0][0]) for _ in range(33)]
+    ws, calls = None, []
+    for i, out in enumerate(outs):
+        q, k, v = sets[i % 3]
+        sel = L.SelectArgs(L.VA_BF16, 1, heads, kv, nq, s, 128, pq, bk, 1, causal, causal, 64, 0, avg[i % 3].data_ptr(), _t4(k),
+                           0.2, None, 0, count.data_ptr(), index.data_ptr(), cap, status.data_ptr(), 0, None, 0)
+        if ws is None:
+            nbytes = C.c_size_t(0)
+            _check(L.lib().va_select_workspace_bytes(C.byref(sel), C.byref(nbytes)))
+            ws = torch.empty(nbytes.value, dtype=torch.uint8, device=DEV)
+        sel.workspace, sel.workspace_bytes = ws.data_ptr(), ws.numel()
+        calls.append((sel, L.AttnArgs(L.VA_BF16, 1, heads, kv, s, s, 128, pq, causal, 0, _t4(q), _t4(k), _t4(v), _t4(out), bcnt.data_ptr(),
+                                      bidx.data_ptr(), bidx.shape[-1], count.data_ptr(), index.data_ptr(), cap, 0.0, status.data_ptr(),
+                                      None, 0, 0, 0)))
+    torch.cuda.synchronize()
+    for i, (sel, att) in enumerate(calls):
+        _check(L.lib().va_select(C.byref(sel), _stream()))
+        _check(L.lib().va_sparse_attn(C.byref(att), _stream()))
+        if i < 3:  # alone
+            torch.cuda.synchronize()
+    torch.cuda.synchronize()
+    assert status.item() == 0 and not torch.equal(outs[0], outs[1])
+    for i, out in enumerate(outs):
+        assert torch.equal(out, outs[i % 3])
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("heads,kv,s", [(300, 100, 200), (40, 40, 1400), (30, 5, 1281)])
 def test_dense_tiles_that_follow_one_another(dtype, heads, kv, s):

@@ -168,6 +168,20 @@ def test_product_package_does_not_import_the_oracle():
                 assert "oracle" not in text.replace("CPU oracle uses the same association", ""), f
 
 
+def test_kernels_that_overlap_their_predecessor_load_coherently():
+    """A kernel that may start while the one before it is still writing must not read through the read-only path, which is
+    for data that nobody writes during the kernel's life."""
+    csrc = os.path.join(ROOT, "vecattention_b200", "csrc")
+    seen = set()
+    for f in os.listdir(csrc):
+        text = re.sub(r"//.*", "", open(os.path.join(csrc, f)).read())
+        if "wait_for_previous();" in text:
+            seen.add(f)
+            assert not re.search(r"__ldg\b|\bldg_nc\b|\.nc\b|__restrict__", text), f
+    assert seen == {"va_select.cu", "va_attn64.cu", "va_attn128.cu", "va_dense128.cu"}
+    assert ".nc" not in re.sub(r"//.*", "", open(os.path.join(csrc, "va_common.cuh")).read())
+
+
 def test_host_pipeline_slices_cover_whole_kv_groups(built_library):
     from vecattention_b200.hostio import head_slices, transfer_bytes
     for heads, kv, n in [(32, 32, 8), (28, 4, 8), (12, 4, 5), (8, 8, 1), (6, 2, 3)]:

@@ -81,8 +81,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
   const int hkv = h / p.rep;
   const int row0 = tile * PQ, row_end = p.sq;  // rows at or past row_end do not exist
   const int64_t trow = ((int64_t)b * p.heads + h) * p.nq + tile;
-  const int nblk = p.own_blocks ? own_block_count<PQ>(p, tile) : (p.blk_count ? __ldg(p.blk_count + trow) : 0);
-  const int ncol = __ldg(p.col_count + trow);
+  const int nblk = p.own_blocks ? own_block_count<PQ>(p, tile) : (p.blk_count ? load_here(p.blk_count + trow) : 0);
+  const int ncol = load_here(p.col_count + trow);
   const int nslots = nblk * 64 + ncol;
   const int nchunks = (nslots + kChunk - 1) / kChunk;
   T* ob = static_cast<T*>(p.out) + b * p.o_sb + h * p.o_sh;
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn128_kernel(const AttnParams p
       const int slot = j * kChunk + my_slot;
       const int ci = min(max(slot - nblk * 64, 0), max(ncol - 1, 0));
       if (p.own_blocks && slot < nblk * 64) return own_block_start<PQ>(p, tile, slot >> 6);
-      return ldg_nc(slot < nblk * 64 ? blk + (slot >> 6) : col + ci);
+      return load_here(slot < nblk * 64 ? blk + (slot >> 6) : col + ci);
     };
     auto decode = [&](int j, int raw) -> int {
       const int slot = j * kChunk + my_slot;

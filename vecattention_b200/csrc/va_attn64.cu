@@ -212,18 +212,18 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn64_kernel(const AttnPa
           int raw[8];
           // requested before the counts are known; a tile with dense blocks, which come first in slot order, fetches again
 #pragma unroll
-          for (int i = 0; i < 8; ++i) raw[i] = !dense && i * 32 + lane < p.col_stride ? ldg_nc(col + i * 32 + lane) : 0;
+          for (int i = 0; i < 8; ++i) raw[i] = !dense && i * 32 + lane < p.col_stride ? load_here(col + i * 32 + lane) : 0;
           const int nblk = dense ? (row_end - 1) / 64 + 1
-                                 : (p.own_blocks ? own_block_count<PQ>(p, tile) : (p.blk_count ? __ldg(p.blk_count + trow) : 0));
-          const int ncol = dense ? 0 : __ldg(p.col_count + trow);
+                                 : (p.own_blocks ? own_block_count<PQ>(p, tile) : (p.blk_count ? load_here(p.blk_count + trow) : 0));
+          const int ncol = dense ? 0 : load_here(p.col_count + trow);
           if (nblk > 0) {
             const int32_t* blk = dense ? nullptr : p.blk_idx + trow * p.blk_stride;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int slot = i * 32 + lane, ci = slot - nblk * 64;
               if (slot < nblk * 64)
-                raw[i] = dense ? (slot >> 6) << 6 : (p.own_blocks ? own_block_start<PQ>(p, tile, slot >> 6) : ldg_nc(blk + (slot >> 6)));
-              else raw[i] = ci < ncol ? ldg_nc(col + ci) : 0;
+                raw[i] = dense ? (slot >> 6) << 6 : (p.own_blocks ? own_block_start<PQ>(p, tile, slot >> 6) : load_here(blk + (slot >> 6)));
+              else raw[i] = ci < ncol ? load_here(col + ci) : 0;
             }
           }
 #pragma unroll
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn64_kernel(const AttnPa
           if (plain) {
             key = (slot < ncol && (unsigned)raw0 < (unsigned)p.sk) ? raw0 : -1;
             raw0 = raw1;
-            if (j + 2 < nchunks) raw1 = ldg_nc(col + min(slot + 2 * kChunk, ncol - 1));
+            if (j + 2 < nchunks) raw1 = load_here(col + min(slot + 2 * kChunk, ncol - 1));
           } else {
             key = slot < nblk * 64 ? raw0 + (slot & 63) : (slot < nblk * 64 + ncol ? raw0 : -1);
             if ((unsigned)key >= (unsigned)p.sk) key = -1;
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_attn64_kernel(const AttnPa
                 raw1 = (s2 >> 6) << 6;  // a dense tile: block i starts at key 64 i
               } else {
                 const int ci = min(max(s2 - nblk * 64, 0), max(ncol - 1, 0));
-                raw1 = ldg_nc(s2 < nblk * 64 ? blk + (s2 >> 6) : col + ci);
+                raw1 = load_here(s2 < nblk * 64 ? blk + (s2 >> 6) : col + ci);
               }
             }
           }

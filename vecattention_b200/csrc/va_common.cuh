@@ -96,10 +96,10 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
-// read-only 32-bit load that the compiler keeps where it is written (used to batch index loads)
-__device__ __forceinline__ int ldg_nc(const int32_t* p) {
+// 32-bit load that the compiler keeps where it is written (used to batch index loads)
+__device__ __forceinline__ int load_here(const int32_t* p) {
   int v;
-  asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 
@@ -118,7 +118,9 @@ inline bool succeeded(cudaError_t e) {
 // A kernel launched with launch_after may be scheduled while the kernel before it in the stream is still running, once
 // every CTA of that one has let it (let_next_start) or ended.  It must not touch memory, not even read an argument's target, and
 // no CTA of it may end before wait_for_previous, which returns when the kernel before has ended and its writes are visible:
-// so the order of all effects is that of plain launches, also for the kernels after it.  What overlaps is the launch itself
+// so the order of all effects is that of plain launches, also for the kernels after it.
+// Such a kernel reads global memory with coherent loads only: not with __ldg or ld.global.nc, which are for data that nobody writes
+// while the kernel lives, and its life begins while the kernel before it is still writing.  What overlaps is the launch itself
 // and the setting up before the wait (barriers, tensor memory).
 // A call that is waited for: 4 heads x 2048 tokens 62.0 -> 57.2 us, 28/4 heads x 9001 360 -> 354, 20 011 around a vision span 817 -> 810;
 // in a row of calls 34.2 -> 33.5 for the first, which the host limits.

@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
       uint4 w = make_uint4(0, 0, 0, 0);
       if (RR < nrows) {
         const int hh = hkv * p.rep + RR % p.rep, tt = RR / p.rep;
-        w = __ldg(reinterpret_cast<const uint4*>(aq + (((int64_t)b * p.heads + hh) * p.nq + tt) * kHeadDim + c * 8));
+        w = *reinterpret_cast<const uint4*>(aq + (((int64_t)b * p.heads + hh) * p.nq + tt) * kHeadDim + c * 8);
         uint32_t* ww = reinterpret_cast<uint32_t*>(&w);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kThreads, 1) select_mask_kernel(const __grid_c
     a.hi = hi;
     a.G = p.group_k_block;
     a.starts = p.starts;
-    a.gap = p.gaps ? __ldg(p.gaps + b * p.gaps_sb + h) : p.gap;
+    a.gap = p.gaps ? p.gaps[b * p.gaps_sb + h] : p.gap;
     a.mrow = p.mask + ((size_t)(b * p.kv_heads + hkv) * p.rows_pad + row_base + wrow) * p.wpad;
     timed_out = !walk_rows<BK, GROUPS>(a, bars, wsh, warp & 3, warp >> 2, lane);
   }
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32) select_expand_kernel(const 
   const int R = tile * p.rep + h % p.rep;
   const int lo = p.wo_initial ? p.pq : 0;
   const int hi = row_key_limit(p, tile, BK);
-  const uint32_t* mrow = p.mask + ((size_t)(b * p.kv_heads + hkv) * p.rows_pad + R) * p.wpad;
+  const int32_t* mrow = reinterpret_cast<const int32_t*>(p.mask) + ((size_t)(b * p.kv_heads + hkv) * p.rows_pad + R) * p.wpad;
   int32_t* out = p.col_idx + row * p.capacity;
   int32_t* stage = stage_s[warp];
   const bool wide = ((p.capacity & 3) | (reinterpret_cast<uintptr_t>(p.col_idx) & 15)) == 0;  // 16-byte stores are possible
@@ -557,9 +557,9 @@ __global__ void __launch_bounds__(kExpandWarps * 32) select_expand_kernel(const 
   if (hi > lo) {
     const int w_hi = (hi + 31) >> 5;
     int w = (lo >> 5) + lane;  // this lane's word
-    uint32_t cur = w < w_hi ? __ldg(mrow + w) : 0u;
+    uint32_t cur = w < w_hi ? (uint32_t)load_here(mrow + w) : 0u;
     for (; w - lane < w_hi; w += 32) {
-      const uint32_t nxt = w + 32 < w_hi ? __ldg(mrow + w + 32) : 0u;  // the next step's words, fetched early
+      const uint32_t nxt = w + 32 < w_hi ? (uint32_t)load_here(mrow + w + 32) : 0u;  // the next step's words, fetched early
       uint32_t word = cur;
       const int c = __popc(word), incl = warp_prefix_sum(c);
       // The lane's keys, last one first: the highest set bit is one instruction of the special-function unit, the lowest
