@@ -151,6 +151,17 @@ def test_python_mirror_raises_like_the_reference(built_library):
         va.average_vector(q, 64)
 
 
+@pytest.mark.parametrize("threshold", [0.5, torch.full((2,), 0.5)])
+def test_vision_composition_checks_its_arguments_before_the_device_is_entered(built_library, threshold):
+    from vecattention_b200 import VecAttention_prefill_vision
+    from vecattention_b200.api import VecAttentionArgumentError
+    q = torch.zeros(1, 2, 256, 128, dtype=torch.bfloat16)
+    with pytest.raises(VecAttentionArgumentError, match="chunk_size"):
+        VecAttention_prefill_vision(q, q, q, threshold, 64, 16, 16, True, 100, vision_start_position=10, vision_end_position=200)
+    with pytest.raises(RuntimeError, match="no CPU fallback"):
+        VecAttention_prefill_vision(q, q, q, threshold, 64, 16, 16, True, 1024, vision_start_position=10, vision_end_position=200)
+
+
 def test_missing_library_fails_loudly(monkeypatch, built_library):
     from vecattention_b200 import _lib
     monkeypatch.setattr(_lib, "_LIB", None)

@@ -17,8 +17,8 @@ from typing import Optional, Tuple, Union
 
 import torch
 
-from .api import (VecAttention_prefill, VecAttentionArgumentError, _gap_of, _sparse_attn_bhsd, average_vector, block_tables,
-                  fuse_qk_softmax_minp_wo_causal)
+from .api import (VecAttention_prefill, VecAttentionArgumentError, _gap_of, _require_cuda, _sparse_attn_bhsd, average_vector,
+                  block_tables, fuse_qk_softmax_minp_wo_causal)
 
 _DENSE_TILE = 64  # query rows per tile of the dense passes
 
@@ -96,9 +96,9 @@ def VecAttention_prefill_vision(
         # shows in the rows the causal rule treats specially), then one attention launch over all rows
         if threshold is None:
             raise VecAttentionArgumentError("threshold is required")
-        gap = _gap_of(threshold, query_states.device)
         if chunk_size % q_pooling_size != 0:
             raise VecAttentionArgumentError("chunk_size must be a multiple of q_pooling_size")
+        gap = _gap_of(threshold, _require_cuda(query_states, key_states, value_states))
         avg = average_vector(query_states[:, :, :end], 64)
         cnt, idx = fuse_qk_softmax_minp_wo_causal(avg, key_states[:, :, :end], 0, gap, True, 64, k_local_size,
                                                   wo_initial=True, group_k_block=group_k_block, compat_q1=compat_q1,
