@@ -678,6 +678,25 @@ static void make_plan(SelectParams& p, int batch, int bk) {
   };
   const int longest = length(blocks - 1);
   const int64_t ctas = (int64_t)blocks * pl.heads;
+  // With eight uncut blocks and more for every SM there is nothing to gain.  The search is made on every call: it takes the blocks'
+  // lengths from their sums, not block by block (causal, host time: 28/4 heads x 64 K, 56 blocks a KV head, 20 -> 4 us; 64/1 x 131 072, 1024 blocks, 244 -> 9).
+  constexpr int kMostBlocks = 2048;
+  const bool search = ctas < 8 * (int64_t)sms && blocks <= kMostBlocks;
+  int64_t total[kMostBlocks + 1];  // tiles of the blocks before
+  if (search && p.causal) {
+    total[0] = 0;
+    for (int i = 0; i < blocks; ++i) total[i + 1] = total[i] + length(i);
+  }
+  // (lengths grow with the block) the first block, not before `from`, of at least n tiles
+  auto first_of = [&](int n, int from) {
+    int lo = from, hi = blocks;
+    while (lo < hi) {
+      const int mid = (lo + hi) / 2;
+      if ((search ? (int)(total[mid + 1] - total[mid]) : length(mid)) < n) lo = mid + 1;
+      else hi = mid;
+    }
+    return lo;
+  };
   // segment s of a block that is cut into n: equal ones where a group starts every few tiles; else each is shorter than the
   // one before by what it walks again, so that all take the same time
   auto set_cuts = [&](int n) {
@@ -715,13 +734,20 @@ static void make_plan(SelectParams& p, int batch, int bk) {
       return (double)((n + sms - 1) / sms) * most;
     }
     int64_t filled = 0;
-    for (int i = 0; i < blocks; ++i) {
-      const int tiles = length(i);
-      for (int s = 0; s < pl.segments && pl.cut[s] < tiles; ++s, n += pl.heads) {
-        const double c = segment_cost(s, tiles);
+    for (int s = 0, reach = 0, fill = 0; s < pl.segments; ++s) {
+      reach = first_of(pl.cut[s] + 1, fill);  // the first block that reaches into the segment, and the first that fills it
+      fill = first_of(pl.cut[s + 1], reach);
+      n += (int64_t)(blocks - reach) * pl.heads;
+      if (fill < blocks) {
+        const double c = segment_cost(s, pl.cut[s + 1]);
         most = c > most ? c : most;
-        sum += c * pl.heads;
-        if (tiles >= pl.cut[s + 1]) filled += pl.heads;
+        sum += c * (blocks - fill) * pl.heads;
+        filled += (int64_t)(blocks - fill) * pl.heads;
+      }
+      if (reach < fill) {
+        const double c = segment_cost(s, length(fill - 1));
+        most = c > most ? c : most;
+        sum += ((double)(total[fill] - total[reach]) + (segment_cost(s, pl.cut[s]) - pl.cut[s]) * (fill - reach)) * pl.heads;
       }
     }
     // the segments that are filled come first, the others fill the gaps
@@ -733,7 +759,7 @@ static void make_plan(SelectParams& p, int batch, int bk) {
   int64_t best_whole = 0;
   double least = 0.0;
   for (const int n : kTry) {
-    if (n > 1 && (n > longest || ctas >= 8 * (int64_t)sms)) break;
+    if (!search || (n > 1 && n > longest)) break;
     set_cuts(n);
     const double c = cost(0);
     if (n == 1 || c < 0.97 * least) {
@@ -763,12 +789,10 @@ static void make_plan(SelectParams& p, int batch, int bk) {
     for (int s = 0; s < pl.segments; ++s) run_of((int)(ctas - best_whole), 0);
   } else {
     int reach[kMaxSegments], fill[kMaxSegments];  // the first block that reaches into segment s, and the first that fills it
-    for (int s = 0, i = 0, j = 0; s < pl.segments; ++s) {
-      while (i < blocks && length(i) <= pl.cut[s]) ++i;
-      while (j < blocks && length(j) < pl.cut[s + 1]) ++j;
-      reach[s] = i;
-      fill[s] = j;
-      run_of(blocks - j, blocks - 1);
+    for (int s = 0; s < pl.segments; ++s) {
+      reach[s] = first_of(pl.cut[s] + 1, 0);
+      fill[s] = first_of(pl.cut[s + 1], 0);
+      run_of(blocks - fill[s], blocks - 1);
     }
     for (int s = 0; s < pl.segments; ++s) run_of(fill[s] - reach[s], fill[s] - 1);
   }
