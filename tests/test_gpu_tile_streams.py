@@ -163,7 +163,8 @@ def test_groups_of_heads(heads, kv, s, causal):
     (14, 2, 20011, 64, 16, 100, True),  # ... every 25th, longer than some segments
     (28, 4, 9001, 64, 16, 8192, True),  # one group: segments walk all keys before them
     (3, 3, 30000, 64, 16, 8192, False),
-    (40, 20, 5000, 64, 64, 2, False),   # whole waves and a cut rest
+    (40, 20, 5000, 64, 64, 2, False),   # 40 row blocks in three segments each
+    (80, 20, 16000, 64, 16, 16, False), # 160 row blocks: a whole wave on 148 SMs, and the other 12 in eleven segments each
     (4, 4, 9000, 128, 128, 1, True),
     (4, 2, 9000, 128, 64, 4, True),
 ])
@@ -264,6 +265,45 @@ def test_selection_and_attention_in_a_row_on_the_same_buffers(pq, bk, causal):
     assert status.item() == 0 and not torch.equal(outs[0], outs[1])
     for i, out in enumerate(outs):
         assert torch.equal(out, outs[i % 3])
+
+
+@pytest.mark.parametrize("what", ["dense", "vision", "operator"])
+def test_calls_right_behind_the_kernels_that_write_their_inputs(what):
+    """Inputs written by the launches just before the call, in the same stream, and in a captured call that starts behind an
+    event of the stream in which they are written."""
+    from vecattention_b200 import VecAttention_prefill, VecAttention_prefill_vision
+    from vecattention_b200.dispatch import Full_prefill
+    call = {"dense": lambda q, k, v: Full_prefill(q, k, v),
+            "vision": lambda q, k, v: VecAttention_prefill_vision(q, k, v, 0.8, 64, 16, 16, True, 16384, vision_start_position=100,
+                                                                  vision_end_position=1300),
+            "operator": lambda q, k, v: VecAttention_prefill(q, k, v, 0.8, 64, 16, 16, True, 16384)}[what]
+    g = torch.Generator(device=DEV).manual_seed(3)
+    sets = [[torch.randn(1, n, 1500, 128, generator=g, device=DEV).bfloat16() for n in (6, 2, 2)] for _ in range(3)]
+    alone = []
+    for x in sets:
+        alone.append(call(*x))
+        torch.cuda.synchronize()
+    x, got = [torch.empty_like(t) for t in sets[0]], []
+    for i in range(30):
+        for a, b in zip(x, sets[i % 3]):
+            torch.add(b, 0.0, out=a)
+        got.append(call(*x))
+    for i, o in enumerate(got):
+        assert torch.equal(o, alone[i % 3])
+    source = [t.clone() for t in sets[0]]
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph):
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            for a, b in zip(x, source):
+                torch.add(b, 0.0, out=a)
+        torch.cuda.current_stream().wait_stream(side)
+        out = call(*x)
+    for i in (1, 2, 0, 2):
+        for a, b in zip(source, sets[i]):
+            a.copy_(b)
+        graph.replay()
+        assert torch.equal(out, alone[i])
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
