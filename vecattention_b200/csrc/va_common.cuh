@@ -118,10 +118,10 @@ inline bool succeeded(cudaError_t e) {
 // A kernel launched with launch_after may be scheduled while the kernel before it in the stream is still running, once
 // every CTA of that one has let it (let_next_start) or ended.  It must not touch memory, not even read an argument's target, and
 // no CTA of it may end before wait_for_previous, which returns when the kernel before has ended and its writes are visible:
-// so the order of all effects is that of plain launches, also for the kernels after it.
+// so the order of all effects is that of plain launches, also for the kernels after it.  What overlaps is the launch itself and, in the
+// 64-row and the dense kernel, the setting up before the wait (barriers, tensor memory).
 // Such a kernel reads global memory with coherent loads only: not with __ldg or ld.global.nc, which are for data that nobody writes
-// while the kernel lives, and its life begins while the kernel before it is still writing.  What overlaps is the launch itself
-// and the setting up before the wait (barriers, tensor memory).
+// while the kernel lives, and its life begins while the kernel before it is still writing.
 // A call that is waited for: 4 heads x 2048 tokens 62.0 -> 57.2 us, 28/4 heads x 9001 360 -> 354, 20 011 around a vision span 817 -> 810;
 // in a row of calls 34.2 -> 33.5 for the first, which the host limits.
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -22,7 +22,7 @@
 // What bounds it: the softmax groups (64 + 128 special-function and fp32 issue slots per score pair and the tensor-memory
 // latencies between them; both groups of a scheduler share its special-function unit).  28 query heads on 4 KV heads, 8192 tokens,
 // whole call: 0.855 ms on gathered 64-row tiles, 0.487-0.503 with a CTA per tile, which set up, filled and drained its pipeline 12 times
-// per SM and whose softmax warps wrote the results, now 0.454-0.471; 16 heads x 500 tokens 42.2 -> 29.8 us, 32/8 heads x 3000 104 -> 84,
+// per SM and whose softmax warps wrote the results, now 0.45-0.47; 16 heads x 500 tokens 42.2 -> 29.8 us, 32/8 heads x 3000 104 -> 84,
 // 16 heads x 16 384 1070 -> 1042.
 #include "va_common.cuh"
 #include "va_sm100.cuh"

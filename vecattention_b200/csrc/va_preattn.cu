@@ -106,8 +106,8 @@ __device__ __forceinline__ void turn(const float (&y)[8], const float (&c)[4], c
 // memory, which one CTA per row with one piece or two per thread in flight was not (2.4 TB/s).  A CTA holds as many
 // whole rows as fit eight warps.
 // Bound by issue slots (71 %), and a row has only sixteen pairs per lane: what is done once a row counts.  With a 64-bit remainder, two
-// divisions by W and a loop over the row's partial sums it took 0.813 ms at 40 heads x 75 600 tokens in bf16 (0.843 in fp16), without
-// them 0.714 (0.725), 4.3 TB/s; 12 heads x 30 000 0.114 -> 0.103.
+// divisions by W and a loop over the row's partial sums it took 0.814-0.818 ms at 40 heads x 75 600 tokens in bf16, without
+// them 0.713-0.741 (eight runs on several GPUs), 4.2-4.4 TB/s; fp16 0.843 -> 0.725, 12 heads x 30 000 tokens 0.114 -> 0.103 (one run each).
 constexpr int NP = 4;  // pieces per lane
 // ROTATE: the call has tables.  The norm alone is a kernel of its own: with the rotation's registers and branches around it,
 // it took 0.612 ms (0.579 before the rotation was done in fp32), alone 0.521 (40 heads, 75 600 tokens).

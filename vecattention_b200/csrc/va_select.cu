@@ -28,10 +28,10 @@
 //                 tcgen05.mma, into one of four 128-column accumulator buffers in tensor memory.
 //    What bounds it: the walkers' instructions, some 500 a tile and scheduler beside 518 clk of tensor arithmetic, of which the
 //    ALU takes two clk each (64 three-input maxima, 64 byte permutes and logic operations).  A tile takes about 1060 clk.
-//    Sixteen warps that read their estimates from tensor memory twice, 96 registers each, spilled; launches then and now:
-//    k_local_size 128 (32 heads x 32 K, causal) 210 -> 122 us; 16: 32 heads x 32 K 168 -> 153, 28/4 heads x 64 K causal 316 -> 286,
-//    9001 tokens, groups of one block, 48 -> 42.  (A funnel shift per estimate in place of conversion, permute and
-//    logic: 1-3 % slower.)
+//    Sixteen warps that read their estimates from tensor memory twice, 96 registers each, spilled.  What eight that hold their row gave,
+//    by themselves: k_local_size 128 (32 heads x 32 K, causal) 210 -> 122 us; 16: 32 heads x 32 K 168 -> 153, 28/4 heads x 64 K causal
+//    316 -> 286, 9001 tokens, groups of one block, 48 -> 42.  With the work cut by make_plan besides, a launch takes 69, 151, 276 and 15 us.
+//    (A funnel shift per estimate in place of conversion, permute and logic: 1-3 % slower.)
 //    All hand-offs are mbarriers with bounded waits; a timeout sets VA_STATUS_TIMEOUT.
 //
 // 2. select_expand_kernel: one warp per pooled row turns the row's keep bits into its ascending
@@ -646,9 +646,15 @@ size_t select_workspace_bytes(int batch, int heads, int kv_heads, int nq, int sk
 // Cut the work into CTAs so that the SMs finish together: the number of segments per row block is the one with the least
 // estimated time, in tiles.  A tile that only feeds the running maximum costs kFeed of one with keep bits (more than its
 // instructions' share: with many segments the CTAs stream K from L2 at the same time), a CTA kSetUp tiles
-// (it loads its rows, fills and drains its pipeline: 3 us).  Whole calls of one group with 0.55 / 0.62 / 0.70: 3 heads x 55 000 tokens 1185 /
-// 1159 / 1112 us, 4 x 55 000 1439 / 1425 / 1414, 5 x 75 600 2629 / 2622 / 2624, 3 x 118 800 3222 / 3203 / 3242 (1167, 1445, 2680 and 3309 with up to four equal
-// segments).
+// (it loads its rows, fills and drains its pipeline: 3 us).
+// Each constant here and below was timed against others, selections alone, on shapes of 1 to 40 heads and 2 to 120 K tokens that the
+// other value cuts differently; time with it / with this one, mean and worst:
+//   kFeed 0.55: 0.98, 1.46 and 0.62: 0.98, 1.47 (some 450 shapes; level from 200 us on; the worst are 40 heads x 9001 and 20 011 tokens,
+//     causal, one group), 0.85: 1.07, 1.14.  Whole calls, not causal, one group, 3 x 55 000 to 3 x 118 800 tokens: level with all three, runs differ by 3-5 %.
+//   kSetUp 2: 1.03, 1.22; 10: 0.99, 1.05 (this and the rest: 14 shapes each).
+//   Another cut is taken if it wins by 3 %, which is what the estimate is good for: by anything 1.04, 1.49; by 10 % 1.01, 1.06.
+//   Work that is spread over the SMs ends 0.2 of the longest CTA after an even share: 0 of it 1.11, 1.29; 0.5 1.01, 1.14.
+//   Segments are whole groups if that makes them at most a quarter longer: only if not at all 1.42, 3.5; up to twice as long 1.02, 1.22.
 static void make_plan(SelectParams& p, int batch, int bk) {
   constexpr double kFeed = 0.70, kSetUp = 5.0;
   Plan& pl = p.plan;
